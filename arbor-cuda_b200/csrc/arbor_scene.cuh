@@ -294,8 +294,10 @@ __device__ __forceinline__ float tube_t(f3 ro, f3 rd, f3 a, f3 b, float ra, floa
   return best;
 }
 // Wood hit (Arbor.cu:192-202): mean-radius tube for shadow rays, bounded
-// SDF march seeded by the analytic tube for primary rays.
-static __device__ __noinline__ float wood_t(const float* P, int id, f3 ro, f3 rd, float footprint, bool refine) {
+// SDF march seeded by the analytic tube for primary rays.  The march only
+// advances from the tube's hit, so one that starts beyond `best` cannot beat
+// it and is not run (the result then only has to be above best).
+static __device__ __noinline__ float wood_t(const float* P, int id, f3 ro, f3 rd, float footprint, bool refine, float best) {
   if (!refine) {
     ARBOR_COUNT(kEvWoodShadow);
     float4 r0 = ldg4(P, id * 6 + 0), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2);
@@ -307,7 +309,7 @@ static __device__ __noinline__ float wood_t(const float* P, int id, f3 ro, f3 rd
   ARBOR_COUNT(kEvWood);
   Wood w = load_wood(P, id);
   float t = tube_t(ro, rd, w.a, w.end, w.ra, w.rb);
-  if (t >= kFar) return kFar;
+  if (t >= kFar || t > best) return kFar;
   f3 lo, hi;
   {
     float r = fmaxf(w.ra, w.rb) + 0.002f;
@@ -391,8 +393,15 @@ __device__ __forceinline__ float leaf_newton(const LeafSolve& s, const LeafShape
     float hy = (leaf_height_parts(u0, yy + e, vp, sh.curl, sh.twist, bw007) - leaf_height_parts(u0, yy - e, vm, sh.curl, sh.twist, bw007)) / (2.0f * e);
     float deriv = dz - hx * dx - hy * dy;
     if (fabsf(deriv) < 0.00001f) break;
+    const float before = t;
     t -= clampf(f / deriv, -0.13f, 0.13f);
     t = clampf(t, s.spanx, s.spany);
+    if (t == before) {
+      // A step is a function of t alone, so every later one would leave it
+      // here too (the work model still counts the reference's seven).
+      for (int j = k + 1; j < 7; j++) ARBOR_COUNT(kEvNewton);
+      break;
+    }
   }
   float xx = x + dx * t;
   float yy = y + dy * t;
@@ -412,7 +421,7 @@ __device__ __forceinline__ float object_t(const float* P, int id, f3 ro, f3 rd, 
   float4 r0 = ldg4(P, id * 6 + 0);
   int type = (int)r0.w;
   if (type < 0) return kFar;
-  if (type == 0) return wood_t(P, id, ro, rd, footprint, refine);
+  if (type == 0) return wood_t(P, id, ro, rd, footprint, refine, kFar);
   if (type == 1) return leaf_t(P, id, ro, rd, footprint, time, wind);
   ARBOR_COUNT(kEvStone);
   f3 h = xyz(ldg4(P, id * 6 + 1));

@@ -44,7 +44,7 @@ struct WarpBatchQ {
   static constexpr int kQ = Q;
   static constexpr int kWarpJobs = 32 * Q;
   float4 rayO[32];             // owner lane's local ray origin and wind time
-  float4 rayD[32];             // owner lane's local ray direction
+  float4 rayD[32];             // owner lane's local ray direction and nearest t so far
   int rayS[32];                // owner lane's scene (forest of several species)
   LeafSolve solve[kNewtonCap];
   int prim[kWarpJobs];         // lane-major queue: lane * Q + k (leaf slot, then record id)
@@ -103,7 +103,7 @@ __device__ __forceinline__ void batch_tests(const TraceCtx& c, const Ray& r, WB&
   const unsigned lt = (1u << lane) - 1u;
   if (nq > 0) {
     b.rayO[lane] = make_float4(r.lro.x, r.lro.y, r.lro.z, r.ltime);
-    b.rayD[lane] = make_float4(r.lrd.x, r.lrd.y, r.lrd.z, 0.0f);
+    b.rayD[lane] = make_float4(r.lrd.x, r.lrd.y, r.lrd.z, r.lbest);
     if (c.species) b.rayS[lane] = r.species;
   }
   // Resolve each queued leaf slot to its record and test class: leaf clip,
@@ -169,6 +169,9 @@ __device__ __forceinline__ void batch_tests(const TraceCtx& c, const Ray& r, WB&
         const float* P = scene_P(c, c.species ? b.rayS[owner] : 0);
         solve = c.refine ? leaf_clip_outlined(P, b.prim[q], mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, c.wind, ls, tube)
                          : leaf_clip(P, b.prim[q], mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, c.wind, ls, tube);
+        // The solve stays inside its clipped interval: one that begins beyond
+        // the owner's nearest t so far cannot beat it.
+        solve = solve && !(ls.spanx > d.w);
         b.res[q] = tube;  // the result, or the Newton stage's starting best
       }
       unsigned m = __ballot_sync(full, solve);
@@ -203,7 +206,7 @@ __device__ __forceinline__ void batch_tests(const TraceCtx& c, const Ray& r, WB&
       int q = b.job[totL + j];
       int owner = q / WB::kQ;
       float4 o = b.rayO[owner], d = b.rayD[owner];
-      b.res[q] = wood_t(scene_P(c, c.species ? b.rayS[owner] : 0), b.prim[q], mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), b.fp[q], true);
+      b.res[q] = wood_t(scene_P(c, c.species ? b.rayS[owner] : 0), b.prim[q], mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), b.fp[q], true, d.w);
     }
   }
   // stones, shadow-ray wood and unused records
