@@ -135,12 +135,13 @@ __device__ __forceinline__ float bark_cut(const Wood& w, f3 p, float fp, float f
   }
   int ix = (int)floorf(x);
   int iy = (int)floorf(y);
+  // columns ix - 1, ix, ix + 1 modulo the column count: one remainder, then
+  // the successors
   int wrapped[3];
-#pragma unroll
-  for (int k = -1; k <= 1; k++) {
-    int cell = ix + k;
-    wrapped[k + 1] = ((cell % w.columns) + w.columns) % w.columns;
-  }
+  wrapped[0] = (ix - 1) % w.columns;
+  if (wrapped[0] < 0) wrapped[0] += w.columns;
+  wrapped[1] = wrapped[0] + 1 == w.columns ? 0 : wrapped[0] + 1;
+  wrapped[2] = wrapped[1] + 1 == w.columns ? 0 : wrapped[1] + 1;
   float first = 100.0f, second = 100.0f;
 #pragma unroll
   for (int j = -1; j <= 1; j++) {
@@ -163,8 +164,12 @@ __device__ __forceinline__ float bark_cut(const Wood& w, f3 p, float fp, float f
   float fissure = 1.0f - smooth(0.015f, 0.17f, gap);
   float plates = fissure * fissure;
   f3 coord = mk(ct * 9.0f, st * 9.0f, arc * 23.0f);
-  float splinter = noise3(coord, w.seed);
-  float pores = noise3(coord * 4.0f, w.seed + 731);
+  // A band past its cut-off footprint has weight 0 and adds a signed zero:
+  // its noise (8 hashes) is not evaluated.  Primary rays: the 2.5 mm band
+  // beyond 2 m, the 10 mm band beyond 8 m at full HD.
+  float splinter = 0.5f, pores = 0.5f;
+  if (fine != 0.0f) splinter = noise3(coord, w.seed);
+  if (grain != 0.0f) pores = noise3(coord * 4.0f, w.seed + 731);
   return amp * clampf(0.32f + coarse * (plates - 0.37f) * 0.69f + fine * (splinter - 0.5f) * 0.24f + grain * (pores - 0.5f) * 0.08f, 0.005f, 1.0f);
 }
 // Wood SDF (Arbor.cu:170).
@@ -297,19 +302,17 @@ __device__ __forceinline__ float tube_t(f3 ro, f3 rd, f3 a, f3 b, float ra, floa
 // SDF march seeded by the analytic tube for primary rays.  The march only
 // advances from the tube's hit, so one that starts beyond `best` cannot beat
 // it and is not run (the result then only has to be above best).
-static __device__ __noinline__ float wood_t(const float* P, int id, f3 ro, f3 rd, float footprint, bool refine, float best) {
-  if (!refine) {
-    ARBOR_COUNT(kEvWoodShadow);
-    float4 r0 = ldg4(P, id * 6 + 0), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2);
-    float p7 = r1.w, p11 = r2.w;
-    float ra = p7 - fminf(0.021f, p7 * 0.055f) * 0.32f;
-    float rb = p11 - fminf(0.021f, p11 * 0.055f) * 0.32f;
-    return tube_t(ro, rd, xyz(r0), xyz(r1), ra, rb);
-  }
-  ARBOR_COUNT(kEvWood);
+//
+// A march can be run a few steps at a time: at most `run` steps are taken from
+// `steps` (0: a new test; else t is the march's place so far).  A finished
+// test returns its result; one that is not returns -t, with `steps` updated.
+static __device__ __noinline__ float wood_run(const float* P, int id, f3 ro, f3 rd, float footprint, float best, float t, int& steps, int run) {
+  if (steps == 0) ARBOR_COUNT(kEvWood);
   Wood w = load_wood(P, id);
-  float t = tube_t(ro, rd, w.a, w.end, w.ra, w.rb);
-  if (t >= kFar || t > best) return kFar;
+  if (steps == 0) {
+    t = tube_t(ro, rd, w.a, w.end, w.ra, w.rb);
+    if (t >= kFar || t > best) return kFar;
+  }
   f3 lo, hi;
   {
     float r = fmaxf(w.ra, w.rb) + 0.002f;
@@ -320,14 +323,24 @@ static __device__ __noinline__ float wood_t(const float* P, int id, f3 ro, f3 rd
   float eps = fmaxf(0.000025f, fminf(0.00025f, footprint * 0.13f));
   float fine = band_weight(0.010f, footprint);
   float grain = band_weight(0.0025f, footprint);
-  for (int k = 0; k < 64; k++) {
+  const int end = min(64, steps + run);
+  for (int k = steps; k < end; k++) {
     ARBOR_COUNT(kEvMarch);
     float f = wood_field<true>(w, ro + rd * t, footprint, fine, grain);
     if (f < eps) return t;
     t += fmaxf(eps * 0.35f, f * 0.27f);
     if (t > span.y) return kFar;
   }
-  return kFar;
+  steps = end;
+  return end == 64 ? kFar : -t;
+}
+__device__ __forceinline__ float wood_shadow_t(const float* P, int id, f3 ro, f3 rd) {
+  ARBOR_COUNT(kEvWoodShadow);
+  float4 r0 = ldg4(P, id * 6 + 0), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2);
+  float p7 = r1.w, p11 = r2.w;
+  float ra = p7 - fminf(0.021f, p7 * 0.055f) * 0.32f;
+  float rb = p11 - fminf(0.021f, p11 * 0.055f) * 0.32f;
+  return tube_t(ro, rd, xyz(r0), xyz(r1), ra, rb);
 }
 // Curved-leaf intersection (Arbor.cu:203-218), in two parts so the
 // wavefront tracer can run them as separate compacted stages: leaf_clip does
@@ -368,10 +381,8 @@ __device__ __forceinline__ bool leaf_clip(const float* P, int id, f3 ro, f3 rd, 
   s.spany = span.y;
   return true;
 }
-// leaf_clip out of line, for the primary-ray passes: a smaller warp loop
-// there (1080p trace 11.0 -> 10.5 ms); the shadow-segment passes keep it
-// inlined (out of line they ran 3x slower).
-static __device__ __noinline__ bool leaf_clip_outlined(const float* P, int id, f3 ro, f3 rd, float time, float wind, LeafSolve& s, float& tube) {
+// leaf_clip out of line, for a rare second call.
+static __device__ __noinline__ bool leaf_clip_again(const float* P, int id, f3 ro, f3 rd, float time, float wind, LeafSolve& s, float& tube) {
   return leaf_clip(P, id, ro, rd, time, wind, s, tube);
 }
 // The Newton stage; `best` is the petiole tube's result.
@@ -416,16 +427,11 @@ static __device__ __noinline__ float leaf_t(const float* P, int id, f3 ro, f3 rd
   if (!leaf_clip(P, id, ro, rd, time, wind, s, tube)) return tube;
   return leaf_newton(s, leaf_shape(P, id), tube, footprint);
 }
-// Arbor.cu:219
-__device__ __forceinline__ float object_t(const float* P, int id, f3 ro, f3 rd, float footprint, float time, float wind, bool refine) {
-  float4 r0 = ldg4(P, id * 6 + 0);
-  int type = (int)r0.w;
-  if (type < 0) return kFar;
-  if (type == 0) return wood_t(P, id, ro, rd, footprint, refine, kFar);
-  if (type == 1) return leaf_t(P, id, ro, rd, footprint, time, wind);
+// Stone ellipsoid (Arbor.cu:219).
+__device__ __forceinline__ float stone_t(const float* P, int id, f3 ro, f3 rd) {
   ARBOR_COUNT(kEvStone);
   f3 h = xyz(ldg4(P, id * 6 + 1));
-  f3 q = ro - xyz(r0);
+  f3 q = ro - xyz(ldg4(P, id * 6));
   f3 p = mk(q.x / h.x, q.y / h.y, q.z / h.z);
   f3 d = mk(rd.x / h.x, rd.y / h.y, rd.z / h.z);
   float aa = dot3(d, d);
@@ -435,6 +441,21 @@ __device__ __forceinline__ float object_t(const float* P, int id, f3 ro, f3 rd, 
   if (disc < 0.0f) return kFar;
   float t = (-bb - sqrtf(disc)) / aa;
   return t > 0.0001f ? t : kFar;
+}
+// Records that are not leaves (Arbor.cu:219): wood (a march of up to `run`
+// steps for primary rays, wood_run), stones, unused ones.
+__device__ __forceinline__ float other_t(const float* P, int id, f3 ro, f3 rd, float footprint, bool refine, float best, float t, int& steps,
+                                         int run) {
+  const int type = (int)ldg4(P, id * 6).w;
+  if (type < 0) return kFar;
+  if (type != 0) return stone_t(P, id, ro, rd);
+  return refine ? wood_run(P, id, ro, rd, footprint, best, t, steps, run) : wood_shadow_t(P, id, ro, rd);
+}
+// Arbor.cu:219
+__device__ __forceinline__ float object_t(const float* P, int id, f3 ro, f3 rd, float footprint, float time, float wind, bool refine) {
+  if ((int)ldg4(P, id * 6).w == 1) return leaf_t(P, id, ro, rd, footprint, time, wind);
+  int steps = 0;
+  return other_t(P, id, ro, rd, footprint, refine, kFar, 0.0f, steps, 64);
 }
 
 // -------------------------------------------------------- traversal --

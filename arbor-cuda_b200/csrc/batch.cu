@@ -5,7 +5,8 @@
 //
 //   batch_setup_kernel        per view: camera constants, the forest
 //                             instance table and the filter/resolve scalars
-//                             of its C record; resets the queues
+//                             of its C record; resets the queues; per scene:
+//                             the tight boxes the passes traverse (tight.cuh)
 //   batch_pool_kernel<trace>  persistent warps walk the views; in each, their
 //                             lanes take pixels from the view's own queue as
 //                             their rays finish and run tracePixels
@@ -46,6 +47,11 @@ namespace {
 // for the shadow pass.
 constexpr int kQueueCompose = 0, kQueueFilter = 1, kViewQueues = 2;
 
+constexpr size_t align256(size_t n) { return (n + 255) / 256 * 256; }
+constexpr size_t kOffP = align256(kB), kOffKeys = kOffP + align256(kP), kOffOrder = kOffKeys + align256(kKeys),
+                 kOffNodes = kOffOrder + align256(kKeys), kOffTight = kOffNodes + align256(kNodes),
+                 kSceneStride = kOffTight + align256(kTightBytes);
+
 struct BatchView {
   const float* P;
   const float* Nodes;
@@ -56,15 +62,26 @@ struct BatchView {
   float* Filtered;
   float* History;
   uint32_t* Pixels;
+  const uint32_t* T;  // the scene's tight boxes (tight.cuh)
   int width, height;
 };
 
+// Blocks 0 .. n_views - 1: one view each; the rest: one part each of the
+// scenes' tight boxes.
 __global__ void __launch_bounds__(kBlock) batch_setup_kernel(const float* __restrict__ Cs, const WorldTrig* __restrict__ trig, Camera* __restrict__ cams,
-                                                             float4* __restrict__ scal, Instance* __restrict__ insts, int* __restrict__ counters) {
+                                                             float4* __restrict__ scal, Instance* __restrict__ insts, int* __restrict__ counters,
+                                                             int n_views, char* scenes) {
   const int v = blockIdx.x;
+  if (v >= n_views) {
+    __shared__ TightPart s;
+    char* base = scenes + (size_t)((v - n_views) / kTightParts) * kSceneStride;
+    tight_build_part(s, (const float*)(base + kOffP), (const uint32_t*)(base + kOffOrder), (const float*)(base + kOffNodes),
+                     (uint32_t*)(base + kOffTight), (v - n_views) % kTightParts);
+    return;
+  }
   if (threadIdx.x == 0) {
     counters[kViewQueues + v] = 0;
-    counters[kViewQueues + gridDim.x + v] = 0;
+    counters[kViewQueues + n_views + v] = 0;
   }
   const float* C = Cs + v * 64;
   if (threadIdx.x == 0) {
@@ -89,9 +106,9 @@ template <int Q, bool kShadow>
 __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* __restrict__ views, const Camera* __restrict__ cams,
                                                                const Instance* __restrict__ insts, const int* __restrict__ list, int n_list,
                                                                int* __restrict__ queues) {
-  using WB = WarpBatchQ<Q>;
+  using BB = BlockBatchOf<Q>;
   extern __shared__ float4 batch_smem[];
-  WB& b = reinterpret_cast<WB*>(batch_smem)[threadIdx.x >> 5];
+  BB& b = *reinterpret_cast<BB*>(batch_smem);
   for (int i = 0; i < n_list; i++) {
     const int v = __ldg(list + i);
     const Camera& cam = cams[v];
@@ -99,15 +116,16 @@ __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* 
     const BatchView view = views[v];
     const int bx = (view.width + 7) / 8;
     const ViewPool pool{queues + v, view.width, view.height, bx, bx * ((view.height + 3) / 4)};
+    const TightView tight = tight_view_warp(view.T, cam.wind);
     Ray r;
     if (kShadow) {
-      const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, 0.0001f, cam.time, cam.wind, false, true};
+      const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, tight, 0.0001f, cam.time, cam.wind, false, true};
       ShadowPolicy policy{&c, &cam, view.Hit, view.Linear, view.width, view.height, 0, 0};
-      batch_run_pool(c, r, b, policy, pool);
+      block_run_pool(c, r, b, policy, pool);
     } else {
-      const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, cam.c14 / (float)view.height, cam.time, cam.wind, true, true};
+      const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, tight, cam.c14 / (float)view.height, cam.time, cam.wind, true, true};
       PrimaryPolicy policy{&cam, view.Hit, view.width, view.height, 0};
-      batch_run_pool(c, r, b, policy, pool);
+      block_run_pool(c, r, b, policy, pool);
     }
   }
 }
@@ -161,7 +179,7 @@ __global__ void __launch_bounds__(kFX * kFT) batch_filter_kernel(const BatchView
 
 template <int Q>
 constexpr size_t batch_smem_bytes() {
-  return sizeof(WarpBatchQ<Q>) * (kBlock / 32);
+  return sizeof(BlockBatchOf<Q>);
 }
 
 int cuda_fail(const char* what, cudaError_t e) {
@@ -174,9 +192,6 @@ int cuda_fail(const char* what, cudaError_t e) {
     if (e_ != cudaSuccess) return cuda_fail(#call, e_); \
   } while (0)
 
-constexpr size_t align256(size_t n) { return (n + 255) / 256 * 256; }
-constexpr size_t kOffP = align256(kB), kOffKeys = kOffP + align256(kP), kOffOrder = kOffKeys + align256(kKeys),
-                 kOffNodes = kOffOrder + align256(kKeys), kSceneStride = kOffNodes + align256(kNodes);
 constexpr int kMaxViews = 65536;
 constexpr int kMaxScenes = 1024;
 
@@ -245,7 +260,8 @@ std::vector<int> view_order(const arbor_batch* b, const std::vector<int>& subset
 }
 
 int launch_setup(arbor_batch* b, cudaStream_t s) {
-  batch_setup_kernel<<<b->n_views, kBlock, 0, s>>>(b->C, world_trig(), b->cams, b->scal, b->insts, b->counters);
+  batch_setup_kernel<<<b->n_views + b->n_scenes * kTightParts, kBlock, 0, s>>>(b->C, world_trig(), b->cams, b->scal, b->insts, b->counters,
+                                                                               b->n_views, b->scenes);
   return check_launch("batch_setup_kernel");
 }
 
@@ -476,7 +492,7 @@ extern "C" int arbor_batch_create(arbor_batch** out, const int* seeds, int n_sce
     char* base = scene_base(b, b->vscene[v]);
     hv[v] = BatchView{(const float*)(base + kOffP), (const float*)(base + kOffNodes), (const uint32_t*)(base + kOffOrder),
                       image(b, 0, v), image(b, 1, v), image(b, 2, v), image(b, 3, v), image(b, 4, v), b->pixels + b->offset[v],
-                      b->vw[v], b->vh[v]};
+                      (const uint32_t*)(base + kOffTight), b->vw[v], b->vh[v]};
     memcpy(b->staging + (size_t)v * 64, views[v].C, kC);
   }
   if ((ce = cudaMemcpyAsync(b->views, hv.data(), hv.size() * sizeof(BatchView), cudaMemcpyHostToDevice, b->own)) != cudaSuccess)

@@ -9,7 +9,7 @@
 // order and every node depend only on + - * / min max of P and are
 // bit-identical to the reference for identical P.
 #include "abi_util.h"
-#include "arbor_scene.cuh"
+#include "tight.cuh"
 
 namespace arbor {
 namespace {
@@ -331,22 +331,6 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(const uint32_t
 }
 
 // ---------------------------------------------------- makeBounds / reduce --
-// Leaf record of one Order slot (Arbor.cu:141): {boundLow, active, boundHigh,
-// id}.  An id outside the 32768 records (invalid input) is given the bounds
-// of an unused record instead of reading out of bounds.
-__device__ __forceinline__ void leaf_record(const float* P, uint32_t uid, float4& lo4, float4& hi4) {
-  if (uid >= (uint32_t)kCapacity) {
-    lo4 = make_float4(kFar, kFar, kFar, 0.0f);
-    hi4 = make_float4(-kFar, -kFar, -kFar, (float)(int)uid);
-    return;
-  }
-  int id = (int)uid;
-  float4 r0 = ldg4(P, id * 6), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2), r4 = ldg4(P, id * 6 + 4);
-  f3 lo, hi;
-  prim_bounds(r0, r1, r1.w, r2.w, r4.x, lo, hi);
-  lo4 = make_float4(lo.x, lo.y, lo.z, r0.w >= 0.0f ? 1.0f : 0.0f);
-  hi4 = make_float4(hi.x, hi.y, hi.z, (float)id);
-}
 __global__ void __launch_bounds__(128) bounds_kernel(const float* __restrict__ P, const uint32_t* __restrict__ Order, float* __restrict__ Nodes) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kCapacity) return;
@@ -355,11 +339,6 @@ __global__ void __launch_bounds__(128) bounds_kernel(const float* __restrict__ P
   float4* n = reinterpret_cast<float4*>(Nodes) + (kCapacity + i) * 2;
   n[0] = lo;
   n[1] = hi;
-}
-// Parent = union of the two children (Arbor.cu:142).
-__device__ __forceinline__ void merge(float4 alo, float4 ahi, float4 clo, float4 chi, float4& plo, float4& phi) {
-  plo = make_float4(fminf(alo.x, clo.x), fminf(alo.y, clo.y), fminf(alo.z, clo.z), alo.w + clo.w);
-  phi = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), -1.0f);
 }
 __global__ void __launch_bounds__(128) reduce_kernel(float* __restrict__ Nodes, int first) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;

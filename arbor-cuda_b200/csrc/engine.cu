@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "abi_util.h"
+#include "scratch.h"
 
 namespace arbor {
 
@@ -73,6 +74,7 @@ struct arbor_engine {
   uint64_t frames = 0;
   arbor_engine_buffers buf{};
   void* scratch = nullptr;
+  uint32_t* tight = nullptr;    // the frame's tight boxes (tight.cuh)
   float* staging = nullptr;  // pinned copy of the input record
   cudaEvent_t input_done = nullptr;
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -214,6 +216,7 @@ extern "C" int arbor_engine_create(arbor_engine** out, int width, int height, in
   if ((ce = cudaMalloc(&e->buf.C, kC)) != cudaSuccess) return fail(cuda_fail("cudaMalloc C", ce));
   if ((ce = cudaMalloc(&e->buf.I, kI)) != cudaSuccess) return fail(cuda_fail("cudaMalloc I", ce));
   if ((ce = cudaMalloc(&e->scratch, arbor_sort_scratch_bytes())) != cudaSuccess) return fail(cuda_fail("cudaMalloc scratch", ce));
+  if ((ce = cudaMalloc(&e->tight, tight_bytes(1))) != cudaSuccess) return fail(cuda_fail("cudaMalloc tight boxes", ce));
   if ((ce = cudaMallocHost(&e->staging, kI)) != cudaSuccess) return fail(cuda_fail("cudaMallocHost input", ce));
   if ((ce = cudaEventCreateWithFlags(&e->input_done, cudaEventDisableTiming)) != cudaSuccess) return fail(cuda_fail("cudaEventCreate", ce));
   for (auto& ev : e->ev)
@@ -285,13 +288,14 @@ extern "C" int arbor_engine_frame(arbor_engine* e, float dt) {
   if (e->timing) ARBOR_CUDA(cudaEventRecord(e->ev[1], s));
   // Visibility (src/engine.js:48)
   if (int r = arbor_updateCamera(b.C, b.I, b.P, delta, e->width, e->height, s)) return r;
-  int r = e->single ? arbor_traceTreePixels(b.P, b.Nodes, b.Order, b.C, b.Hit, e->width, e->height, s)
-                    : arbor_tracePixels(b.P, b.Nodes, b.Order, b.C, b.Hit, e->width, e->height, s);
+  // (the frame's passes share one set of tight boxes, in the engine's own memory)
+  int r = launch_tight(b.P, b.Order, b.Nodes, 1, e->tight, b.C, false, s);
+  if (!r) r = launch_trace("arbor_engine_frame", !e->single, b.P, b.Nodes, b.Order, e->tight, b.C, b.Hit, e->width, e->height, s);
   if (r) return r;
   if (e->timing) ARBOR_CUDA(cudaEventRecord(e->ev[2], s));
   // Materials and light (:49)
-  r = e->single ? arbor_shadeTreePixels(b.P, b.Nodes, b.Order, b.C, b.Hit, b.Linear, b.Guide, e->width, e->height, s)
-                : arbor_shadePixels(b.P, b.Nodes, b.Order, b.C, b.Hit, b.Linear, b.Guide, e->width, e->height, s);
+  r = launch_shade("arbor_engine_frame", !e->single, b.P, b.Nodes, b.Order, e->tight, b.C, b.Hit, b.Linear, b.Guide, nullptr, e->width,
+                   e->height, s);
   if (r) return r;
   if (e->timing) ARBOR_CUDA(cudaEventRecord(e->ev[3], s));
   // Progressive resolve (:50), filter and resolve fused.
@@ -321,8 +325,8 @@ extern "C" int arbor_engine_inspect(arbor_engine* e, arbor_engine_info* info) {
   info->single_tree = e->single ? 1 : 0;
   info->frames = e->frames;
   info->scene_bytes = e->scene_bytes;
-  info->allocated_bytes = e->scene_bytes + kC + kI + arbor_sort_scratch_bytes() + e->image_bytes_total;
-  info->launches_per_frame = 6;  // updateCamera, trace, shadow setup + shadow pass + compose (shadePixels), filterResolve
+  info->allocated_bytes = e->scene_bytes + kC + kI + arbor_sort_scratch_bytes() + tight_bytes(1) + e->image_bytes_total;
+  info->launches_per_frame = 6;  // updateCamera, tight boxes, trace, shadow pass + compose (shadePixels), filterResolve
   info->ms_build = e->ms_build;
   info->ms_visibility = e->ms_vis;
   info->ms_lighting = e->ms_light;
@@ -369,6 +373,8 @@ extern "C" int arbor_engine_dispose(arbor_engine* e) {
   cudaFree(e->buf.C);
   cudaFree(e->buf.I);
   cudaFree(e->scratch);
+  cudaFree(e->tight);
+  e->tight = nullptr;
   e->buf = arbor_engine_buffers{};
   e->scratch = nullptr;
   if (e->staging) cudaFreeHost(e->staging);

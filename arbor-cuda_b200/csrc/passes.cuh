@@ -17,8 +17,8 @@ __device__ __forceinline__ void tile_pixel_at(int t, int x0, int y0, int tw, int
 }
 
 // ---------------------------------------------------------------- trace --
-// Primary rays (tracePixels); each warp's primitive tests run warp-batched
-// (warpbatch.cuh).
+// Primary rays (tracePixels); each block's primitive tests run batched
+// (blockbatch.cuh).
 struct PrimaryPolicy {
   static constexpr int kRefill = 8;  // idle lanes that trigger a refill (measured best of 1-16)
   const Camera* cam;
@@ -43,7 +43,7 @@ template <class WB>
 __device__ __forceinline__ void trace_pool(const TraceCtx& c, const Camera& cam, WB& b, float* __restrict__ Hit, const PixelPool& pool) {
   PrimaryPolicy policy{&cam, Hit, pool.width, pool.height, 0};
   Ray r;
-  batch_run_pool(c, r, b, policy, pool);
+  block_run_pool(c, r, b, policy, pool);
 }
 
 // ---------------------------------------------------------------- shade --
@@ -394,11 +394,11 @@ __device__ __forceinline__ void shadow_pool(const TraceCtx& c, const Camera& cam
                                             const PixelPool& pool) {
   ShadowPolicy policy{&c, &cam, Hit, Vis, pool.width, pool.height, 0, 0};
   Ray r;
-  batch_run_pool(c, r, b, policy, pool);
+  block_run_pool(c, r, b, policy, pool);
 }
 
 // The same shadow segments with each pixel's ray staged in memory by the
-// setup pass (shadow_setup_px): origin in Vis (w = 1 when the pixel has a
+// same CTA (stage_shadows): origin in Vis (w = 1 when the pixel has a
 // shadow ray), direction in Dir.  The tracer's loop then holds no camera or
 // sun-sampling code.
 struct StagedShadowPolicy {
@@ -414,7 +414,7 @@ struct StagedShadowPolicy {
     const float4 o = reinterpret_cast<const float4*>(Vis)[pixel];
     if (o.w == 1.0f) {
       origin = mk(o.x, o.y, o.z);
-      light = xyz(__ldg(reinterpret_cast<const float4*>(Dir) + pixel));
+      light = xyz(reinterpret_cast<const float4*>(Dir)[pixel]);
       trans = mk(1.0f, 1.0f, 1.0f);
       seg = 0;
       ray_begin(c, r, origin, light, 36.0f);
@@ -444,7 +444,7 @@ struct StagedShadowPolicy {
 
 // Stage pixel (x, y)'s shadow ray for StagedShadowPolicy: origin and w = 1
 // into Vis and the direction into Dir, or Vis.w = 0 without a shadow ray.
-__device__ __forceinline__ void shadow_setup_px(const Camera& cam, const float* __restrict__ Hit, float* __restrict__ Vis, float* __restrict__ Dir,
+__device__ __forceinline__ void shadow_setup_px(const Camera& cam, const float* __restrict__ Hit, float* Vis, float* Dir,
                                                 int x, int y, int width, int height) {
   const int pixel = y * width + x;
   f3 origin, light;
@@ -456,13 +456,26 @@ __device__ __forceinline__ void shadow_setup_px(const Camera& cam, const float* 
   }
 }
 
+// Stage the shadow rays of every pixel of a persistent CTA's pool (the pixels
+// pool_take hands out); every thread of the block calls it.
+__device__ __forceinline__ void stage_shadows(const Camera& cam, const float* __restrict__ Hit, float* Vis, float* Dir, const PixelPool& pool) {
+  for (int idx = threadIdx.x;; idx += blockDim.x) {
+    const int block = (int)blockIdx.x + (idx >> 5) * (int)gridDim.x;
+    if (block >= pool.blocks) break;
+    const int by = block / pool.blocks_x, bx = block - by * pool.blocks_x;
+    const int x = bx * 8 + (idx & 7), y = by * 4 + ((idx >> 3) & 3);
+    if (x < pool.width && y < pool.height) shadow_setup_px(cam, Hit, Vis, Dir, x, y, pool.width, pool.height);
+  }
+  __syncthreads();
+}
+
 // Staged shadow segments of every pixel of a persistent CTA's pool.
 template <class WB>
-__device__ __forceinline__ void staged_shadow_pool(const TraceCtx& c, WB& b, const float* __restrict__ Dir, float* __restrict__ Vis,
+__device__ __forceinline__ void staged_shadow_pool(const TraceCtx& c, WB& b, const float* Dir, float* Vis,
                                                    const PixelPool& pool) {
   StagedShadowPolicy policy{&c, Dir, Vis, pool.width, pool.height, 0, 0};
   Ray r;
-  batch_run_pool(c, r, b, policy, pool);
+  block_run_pool(c, r, b, policy, pool);
 }
 
 // shadePixels' colour of pixel (x, y) (Arbor.cu:277-289), its visibility

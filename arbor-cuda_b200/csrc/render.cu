@@ -13,86 +13,102 @@
 
 #include "abi_util.h"
 #include "passes.cuh"
+#include "scratch.h"
 
 namespace arbor {
 namespace {
 
 // ---------------------------------------------------------------- kernels --
+// Dynamic shared memory of a persistent pass: the block batch and, for a pass
+// without scratch, room for an instance table.
+struct PassSmem {
+  BlockBatch batch;
+  Instance table[kForest];
+};
+constexpr size_t kPassSmem = sizeof(BlockBatch), kPassSmemTable = sizeof(PassSmem);
+static_assert(2 * (kPassSmemTable + 1024 + 512) <= 228 * 1024, "two CTAs per SM");
+static_assert(kBlock == kThreads, "a block batch is one block's");
 // The instance table of a persistent pass: the registry slot's (global
-// memory) when the host registered the world seed, else one built in the
-// dynamic shared memory of the CTA's last two warp batches, whose warps then
-// leave (kTableWarps warps trace).  Every thread of the block calls it.
-constexpr int kTableWarps = kBlock / 32 - 2;
-static_assert(2 * sizeof(WarpBatch) >= sizeof(Instance) * kForest, "two warp batches hold an instance table");
-__device__ __forceinline__ const Instance* pass_instances(const WorldTrig* trig, int ws, float4* smem, bool& leave) {
+// memory) when the host registered the world seed, else the one in the
+// scratch behind n_scenes' tight boxes (tight_kernel), or without scratch one
+// built in shared memory.  Every thread of the block calls it.
+__device__ __forceinline__ const Instance* pass_instances(const WorldTrig* trig, int ws, const uint32_t* T, int n_scenes, PassSmem& smem) {
   const WorldTrig* slot = world_slot_of(trig, ws);
-  leave = false;
   if (slot != nullptr) return slot->inst;
-  Instance* table = reinterpret_cast<Instance*>(reinterpret_cast<WarpBatch*>(smem) + kTableWarps);
-  for (int t = threadIdx.x; t < kForest; t += blockDim.x) table[t] = make_instance(t, ws);
+  if (T != nullptr) return reinterpret_cast<const Instance*>(T + (size_t)n_scenes * kTightWords);
+  for (int t = threadIdx.x; t < kForest; t += blockDim.x) smem.table[t] = make_instance(t, ws);
   __syncthreads();
-  leave = (int)(threadIdx.x >> 5) >= kTableWarps;
-  return table;
+  return smem.table;
 }
 
 // Persistent form of the trace: a grid of (SMs x 2) CTAs, each taking every
 // gridDim.x-th 8x4-pixel block of the image, its lanes taking pixels as
-// their rays finish (batch_run_pool).
+// their rays finish (block_run_pool).
 template <bool kForestScene>
 __global__ void __launch_bounds__(kBlock, 2) trace_pool_kernel(const float* __restrict__ P, const float* __restrict__ Nodes,
                                                                const uint32_t* __restrict__ Order, const float* __restrict__ C,
-                                                               const WorldTrig* __restrict__ trig,
+                                                               const WorldTrig* __restrict__ trig, const uint32_t* __restrict__ T,
                                                                float* __restrict__ Hit, int width, int height) {
   extern __shared__ float4 batch_smem[];
-  WarpBatch& b = reinterpret_cast<WarpBatch*>(batch_smem)[threadIdx.x >> 5];
+  PassSmem& smem = *reinterpret_cast<PassSmem*>(batch_smem);
   __shared__ Camera cam;
   __shared__ int next;
   if (threadIdx.x == 0) next = 0;
   block_setup(C, cam, nullptr, false, nullptr);
-  bool leave = false;
-  const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, batch_smem, leave) : nullptr;
-  if (leave) return;
-  const TraceCtx c{P, Nodes, Order, inst, cam.c14 / (float)height, cam.time, cam.wind, true, kForestScene};
+  const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, T, 1, smem) : nullptr;
+  const TightView tight = tight_view_block(T, P, Order, Nodes, 1, cam.wind);
+  const TraceCtx c{P, Nodes, Order, inst, tight, cam.c14 / (float)height, cam.time, cam.wind, true, kForestScene};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
-  trace_pool(c, cam, b, Hit, pool);
+  trace_pool(c, cam, smem.batch, Hit, pool);
 }
 
 // shadePixels in two passes.  The shadow pass is persistent like the trace:
 // lanes take pixels from a pool and trace their shadow segments, writing the
-// visibility into Linear; with sun shadows off it returns at once.
+// visibility into Linear; with sun shadows off it returns at once.  Each CTA
+// first stages the shadow rays of its own pixels (stage_shadows: origin into
+// Linear, direction into Guide; both are overwritten by the compose pass), so
+// the tracer's loop holds no camera or sun-sampling code.
 template <bool kForestScene>
 __global__ void __launch_bounds__(kBlock, 2) shadow_pool_kernel(const float* __restrict__ P, const float* __restrict__ Nodes,
                                                                 const uint32_t* __restrict__ Order, const float* __restrict__ C,
-                                                                const WorldTrig* __restrict__ trig,
-                                                                const float* __restrict__ Guide, float* __restrict__ Linear, int width, int height) {
+                                                                const WorldTrig* __restrict__ trig, const uint32_t* __restrict__ T,
+                                                                const float* __restrict__ Hit, float* Guide, float* Linear, int width, int height) {
   extern __shared__ float4 batch_smem[];
-  WarpBatch& b = reinterpret_cast<WarpBatch*>(batch_smem)[threadIdx.x >> 5];
+  PassSmem& smem = *reinterpret_cast<PassSmem*>(batch_smem);
   __shared__ Camera cam;
   __shared__ int next;
   if (threadIdx.x == 0) next = 0;
   block_setup(C, cam, nullptr, false, nullptr);
   if (!(cam.shadows > 0.5f)) return;
-  bool leave = false;
-  const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, batch_smem, leave) : nullptr;
-  if (leave) return;
-  const TraceCtx c{P, Nodes, Order, inst, 0.0001f, cam.time, cam.wind, false, kForestScene};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
-  staged_shadow_pool(c, b, Guide, Linear, pool);
+  stage_shadows(cam, Hit, Linear, Guide, pool);
+  const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, T, 1, smem) : nullptr;
+  const TightView tight = tight_view_block(T, P, Order, Nodes, 1, cam.wind);
+  const TraceCtx c{P, Nodes, Order, inst, tight, 0.0001f, cam.time, cam.wind, false, kForestScene};
+  staged_shadow_pool(c, smem.batch, Guide, Linear, pool);
 }
 
-// Stages each pixel's shadow ray for the shadow pass (origin into Linear,
-// direction into Guide; both are overwritten by the compose pass); with sun
-// shadows off it returns at once.
-__global__ void __launch_bounds__(kBlock) shadow_setup_kernel(const float* __restrict__ C, const float* __restrict__ Hit, float* __restrict__ Linear,
-                                                              float* __restrict__ Guide, int width, int height) {
-  __shared__ Camera cam;
-  block_setup(C, cam, nullptr, false, nullptr);
-  if (!(cam.shadows > 0.5f)) return;
-  int x, y;
-  tile_pixel_at(threadIdx.x, blockIdx.x * kTile, blockIdx.y * kTile, kTile, x, y);
-  if (x < width && y < height) shadow_setup_px(cam, Hit, Linear, Guide, x, y, width, height);
+// The tight boxes (tight.cuh) of n_scenes scenes, one part per CTA, and behind
+// them, by one more CTA, the instance table of a world seed that the registry
+// does not hold.  C: the pass's camera record; with `shadows` the boxes are
+// for a shadow pass, and with sun shadows off nothing is made.
+__global__ void __launch_bounds__(kBlock) tight_kernel(const float* __restrict__ P, const uint32_t* __restrict__ Order,
+                                                       const float* __restrict__ Nodes, uint32_t* __restrict__ T, int n_scenes,
+                                                       const float* __restrict__ C, bool shadows, const WorldTrig* __restrict__ trig) {
+  __shared__ TightPart s;
+  if (shadows && !(C[22] > 0.5f)) return;
+  const size_t k = blockIdx.x / kTightParts;
+  if ((int)k == n_scenes) {
+    const int ws = (int)C[31];
+    if (world_slot_of(trig, ws) != nullptr) return;
+    Instance* table = reinterpret_cast<Instance*>(T + k * kTightWords);
+    for (int t = threadIdx.x; t < kForest; t += blockDim.x) table[t] = make_instance(t, ws);
+    return;
+  }
+  tight_build_part(s, P + k * (kCapacity * kPS), Order + k * kCapacity, Nodes + k * (kNodeCount * 8), T + k * kTightWords,
+                   (int)(blockIdx.x % kTightParts));
 }
 
 // The compose pass: one pixel per thread, the surface terms and the colour
@@ -130,32 +146,31 @@ __device__ __forceinline__ void species_setup(Instance* inst, const SpeciesMap& 
 
 __global__ void __launch_bounds__(kBlock, 2) trace_species_kernel(const float* __restrict__ P, const float* __restrict__ Nodes,
                                                                   const uint32_t* __restrict__ Order, const float* __restrict__ C,
-                                                                  const WorldTrig* __restrict__ trig,
+                                                                  const WorldTrig* __restrict__ trig, const uint32_t* __restrict__ T, int n_scenes,
                                                                   float* __restrict__ Hit, int width, int height, const SpeciesMap map) {
   extern __shared__ float4 batch_smem[];
-  WarpBatch& b = reinterpret_cast<WarpBatch*>(batch_smem)[threadIdx.x >> 5];
+  PassSmem& smem = *reinterpret_cast<PassSmem*>(batch_smem);
   __shared__ Camera cam;
   __shared__ uint8_t of[kForest];
   __shared__ int next;
   if (threadIdx.x == 0) next = 0;
   for (int t = threadIdx.x; t < kForest; t += blockDim.x) of[t] = map.of[t];
   block_setup(C, cam, nullptr, false, nullptr);
-  bool leave = false;
-  const Instance* inst = pass_instances(trig, cam.ws, batch_smem, leave);
-  if (leave) return;
-  const TraceCtx c{P, Nodes, Order, inst, cam.c14 / (float)height, cam.time, cam.wind, true, true, true, of};
+  const Instance* inst = pass_instances(trig, cam.ws, T, n_scenes, smem);
+  const TightView tight = tight_view_block(T, P, Order, Nodes, n_scenes, cam.wind);
+  const TraceCtx c{P, Nodes, Order, inst, tight, cam.c14 / (float)height, cam.time, cam.wind, true, true, true, of};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
-  trace_pool(c, cam, b, Hit, pool);
+  trace_pool(c, cam, smem.batch, Hit, pool);
 }
 
 __global__ void __launch_bounds__(kBlock, 2) shadow_species_kernel(const float* __restrict__ P, const float* __restrict__ Nodes,
                                                                    const uint32_t* __restrict__ Order, const float* __restrict__ C,
-                                                                   const WorldTrig* __restrict__ trig,
-                                                                   const float* __restrict__ Guide, float* __restrict__ Linear, int width, int height,
+                                                                   const WorldTrig* __restrict__ trig, const uint32_t* __restrict__ T, int n_scenes,
+                                                                   const float* __restrict__ Hit, float* Guide, float* Linear, int width, int height,
                                                                    const SpeciesMap map) {
   extern __shared__ float4 batch_smem[];
-  WarpBatch& b = reinterpret_cast<WarpBatch*>(batch_smem)[threadIdx.x >> 5];
+  PassSmem& smem = *reinterpret_cast<PassSmem*>(batch_smem);
   __shared__ Camera cam;
   __shared__ uint8_t of[kForest];
   __shared__ int next;
@@ -163,13 +178,13 @@ __global__ void __launch_bounds__(kBlock, 2) shadow_species_kernel(const float* 
   for (int t = threadIdx.x; t < kForest; t += blockDim.x) of[t] = map.of[t];
   block_setup(C, cam, nullptr, false, nullptr);
   if (!(cam.shadows > 0.5f)) return;
-  bool leave = false;
-  const Instance* inst = pass_instances(trig, cam.ws, batch_smem, leave);
-  if (leave) return;
-  const TraceCtx c{P, Nodes, Order, inst, 0.0001f, cam.time, cam.wind, false, true, true, of};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
-  staged_shadow_pool(c, b, Guide, Linear, pool);
+  stage_shadows(cam, Hit, Linear, Guide, pool);
+  const Instance* inst = pass_instances(trig, cam.ws, T, n_scenes, smem);
+  const TightView tight = tight_view_block(T, P, Order, Nodes, n_scenes, cam.wind);
+  const TraceCtx c{P, Nodes, Order, inst, tight, 0.0001f, cam.time, cam.wind, false, true, true, of};
+  staged_shadow_pool(c, smem.batch, Guide, Linear, pool);
 }
 
 __global__ void __launch_bounds__(kBlock, 4) shade_compose_species_kernel(const float* __restrict__ P, const float* __restrict__ C,
@@ -279,10 +294,8 @@ __global__ void __launch_bounds__(kRX * kRY) resolve_kernel(const float* __restr
   resolve_px(mk(f.x, f.y, f.z), History, Pixels, count, 1.0f / (count + 1.0f), C[20], vig_coord(x, width), vig_coord(y, height), y * width + x);
 }
 
-// Dynamic shared memory of a 256-thread CTA: one WarpBatch per warp.
-constexpr size_t kBatchSmem = sizeof(WarpBatch) * (kBlock / 32);
 
-// Opt a kernel in to kBatchSmem of dynamic shared memory, once per device.
+// Opt a kernel in to kPassSmemTable of dynamic shared memory, once per device.
 inline bool batch_smem_ready(const void* kernel) {
   static const void* done[64][8] = {};
   int dev = 0;
@@ -290,12 +303,12 @@ inline bool batch_smem_ready(const void* kernel) {
   for (int i = 0; i < 8; i++) {
     if (done[dev][i] == kernel) return true;
     if (done[dev][i] == nullptr) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem) != cudaSuccess) return false;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmemTable) != cudaSuccess) return false;
       done[dev][i] = kernel;
       return true;
     }
   }
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem) == cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmemTable) == cudaSuccess;
 }
 
 dim3 pixel_grid(int w, int h) { return dim3((w + kTile - 1) / kTile, (h + kTile - 1) / kTile); }
@@ -325,27 +338,73 @@ int launch_filter(const char* name, bool resolve, const float* Linear, const flo
 }
 dim3 resolve_grid(int w, int h) { return dim3((w + kRX - 1) / kRX, (h + kRY - 1) / kRY); }
 
-int trace_entry(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const float* C, float* Hit, int width,
-                int height, cudaStream_t stream) {
-  bool empty;
-  if (int s = check_image(name, width, height, &empty)) return s;
+// Checks of tracePixels / shadePixels, shared by the entries and the engine.
+int trace_checks(const char* name, const float* P, const float* Nodes, const uint32_t* Order, const float* C, const float* Hit, int width,
+                 int height, bool* empty) {
+  if (int s = check_image(name, width, height, empty)) return s;
   const Binding b[] = {{P, kP, false, 16, "P"},
                        {Nodes, kNodes, false, 16, "Nodes"},
                        {Order, kKeys, false, 4, "Order"},
                        {C, kC, false, 4, "C"},
-                       {Hit, empty ? 0 : image_bytes(width, height), true, 16, "Hit"}};
-  if (int s = check_bindings(name, b)) return s;
-  if (empty) return ARBOR_OK;
-  if (!batch_smem_ready(forest ? (const void*)trace_pool_kernel<true> : (const void*)trace_pool_kernel<false>)) {
-    set_error("%s: cannot reserve %zu bytes of shared memory per CTA", name, kBatchSmem);
-    return ARBOR_ERR_CUDA;
-  }
+                       {Hit, *empty ? 0 : image_bytes(width, height), true, 16, "Hit"}};
+  return check_bindings(name, b);
+}
+int smem_error(const char* name) {
+  set_error("%s: cannot reserve %zu bytes of shared memory per CTA", name, kPassSmemTable);
+  return ARBOR_ERR_CUDA;
+}
+
+}  // namespace
+
+size_t tight_bytes(int n_scenes) { return kTightBytes * (size_t)n_scenes + sizeof(Instance) * kForest; }
+int launch_tight(const float* P, const uint32_t* Order, const float* Nodes, int n_scenes, uint32_t* T, const float* C, bool shadows,
+                 cudaStream_t stream) {
+  tight_kernel<<<kTightParts * n_scenes + 1, kBlock, 0, stream>>>(P, Order, Nodes, T, n_scenes, C, shadows, world_trig());
+  count_launch();
+  return check_launch("tight_kernel");
+}
+
+// tracePixels over the boxes T (tight boxes of the scene, or null: Nodes).
+int launch_trace(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const uint32_t* T, const float* C,
+                 float* Hit, int width, int height, cudaStream_t stream) {
+  if (!batch_smem_ready(forest ? (const void*)trace_pool_kernel<true> : (const void*)trace_pool_kernel<false>)) return smem_error(name);
   if (forest)
-    trace_pool_kernel<true><<<pool_grid(width, height), kBlock, kBatchSmem, stream>>>(P, Nodes, Order, C, world_trig(), Hit, width, height);
+    trace_pool_kernel<true><<<pool_grid(width, height), kBlock, T ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), T, Hit, width, height);
   else
-    trace_pool_kernel<false><<<pool_grid(width, height), kBlock, kBatchSmem, stream>>>(P, Nodes, Order, C, world_trig(), Hit, width, height);
+    trace_pool_kernel<false><<<pool_grid(width, height), kBlock, T ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), T, Hit, width, height);
   count_launch();
   return check_launch(name);
+}
+
+// shadePixels over the boxes T: shadow segments in a persistent pass whose
+// loop holds only the tracer (its code stays small), then the shading of
+// every pixel.
+int launch_shade(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const uint32_t* T, const float* C,
+                 const float* Hit, float* Linear, float* Guide, float* Normal, int width, int height, cudaStream_t stream) {
+  if (!batch_smem_ready(forest ? (const void*)shadow_pool_kernel<true> : (const void*)shadow_pool_kernel<false>)) return smem_error(name);
+  if (forest) {
+    shadow_pool_kernel<true><<<pool_grid(width, height), kBlock, T ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), T, Hit, Guide, Linear,
+                                                                                       width, height);
+    shade_compose_kernel<true><<<pixel_grid(width, height), kBlock, 0, stream>>>(P, C, world_trig(), Hit, Linear, Guide, Normal, width, height);
+  } else {
+    shadow_pool_kernel<false><<<pool_grid(width, height), kBlock, T ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), T, Hit, Guide, Linear,
+                                                                                        width, height);
+    shade_compose_kernel<false><<<pixel_grid(width, height), kBlock, 0, stream>>>(P, C, world_trig(), Hit, Linear, Guide, Normal, width, height);
+  }
+  count_launch(2);
+  return check_launch(name);
+}
+
+namespace {
+
+int trace_entry(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const float* C, float* Hit, int width,
+                int height, cudaStream_t stream) {
+  bool empty;
+  if (int s = trace_checks(name, P, Nodes, Order, C, Hit, width, height, &empty)) return s;
+  if (empty) return ARBOR_OK;
+  const TightScratch t(P, Order, Nodes, 1, C, false, stream);
+  if (t.status) return t.status;
+  return launch_trace(name, forest, P, Nodes, Order, t.boxes, C, Hit, width, height, stream);
 }
 
 int shade_entry(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const float* C, const float* Hit,
@@ -363,22 +422,9 @@ int shade_entry(const char* name, bool forest, const float* P, const float* Node
     if (int s = check_bindings(name, g)) return s;
   }
   if (empty) return ARBOR_OK;
-  if (!batch_smem_ready(forest ? (const void*)shadow_pool_kernel<true> : (const void*)shadow_pool_kernel<false>)) {
-    set_error("%s: cannot reserve %zu bytes of shared memory per CTA", name, kBatchSmem);
-    return ARBOR_ERR_CUDA;
-  }
-  // Shadow segments in a persistent pass whose loop holds only the tracer
-  // (its code stays small), then the shading of every pixel.
-  shadow_setup_kernel<<<pixel_grid(width, height), kBlock, 0, stream>>>(C, Hit, Linear, Guide, width, height);
-  if (forest) {
-    shadow_pool_kernel<true><<<pool_grid(width, height), kBlock, kBatchSmem, stream>>>(P, Nodes, Order, C, world_trig(), Guide, Linear, width, height);
-    shade_compose_kernel<true><<<pixel_grid(width, height), kBlock, 0, stream>>>(P, C, world_trig(), Hit, Linear, Guide, Normal, width, height);
-  } else {
-    shadow_pool_kernel<false><<<pool_grid(width, height), kBlock, kBatchSmem, stream>>>(P, Nodes, Order, C, world_trig(), Guide, Linear, width, height);
-    shade_compose_kernel<false><<<pixel_grid(width, height), kBlock, 0, stream>>>(P, C, world_trig(), Hit, Linear, Guide, Normal, width, height);
-  }
-  count_launch(3);
-  return check_launch(name);
+  const TightScratch t(P, Order, Nodes, 1, C, true, stream);
+  if (t.status) return t.status;
+  return launch_shade(name, forest, P, Nodes, Order, t.boxes, C, Hit, Linear, Guide, Normal, width, height, stream);
 }
 
 // Checks of a forest-of-species call: 1..256 scenes, every instance on one
@@ -422,11 +468,11 @@ extern "C" int arbor_traceSpeciesPixels(const float* P, const float* Nodes, cons
                        {Hit, empty ? 0 : image_bytes(width, height), true, 16, "Hit"}};
   if (int s = check_bindings(name, b)) return s;
   if (empty) return ARBOR_OK;
-  if (!batch_smem_ready((const void*)trace_species_kernel)) {
-    set_error("%s: cannot reserve %zu bytes of shared memory per CTA", name, kBatchSmem);
-    return ARBOR_ERR_CUDA;
-  }
-  trace_species_kernel<<<pool_grid(width, height), kBlock, kBatchSmem, stream>>>(P, Nodes, Order, C, world_trig(), Hit, width, height, map);
+  if (!batch_smem_ready((const void*)trace_species_kernel)) return smem_error(name);
+  const TightScratch t(P, Order, Nodes, n_species, C, false, stream);
+  if (t.status) return t.status;
+  trace_species_kernel<<<pool_grid(width, height), kBlock, t.boxes ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), t.boxes, n_species, Hit, width,
+                                                                                 height, map);
   count_launch();
   return check_launch(name);
 }
@@ -444,14 +490,13 @@ extern "C" int arbor_shadeSpeciesPixels(const float* P, const float* Nodes, cons
                        {Guide, img, true, 16, "Guide"}};
   if (int s = check_bindings(name, b)) return s;
   if (empty) return ARBOR_OK;
-  if (!batch_smem_ready((const void*)shadow_species_kernel)) {
-    set_error("%s: cannot reserve %zu bytes of shared memory per CTA", name, kBatchSmem);
-    return ARBOR_ERR_CUDA;
-  }
-  shadow_setup_kernel<<<pixel_grid(width, height), kBlock, 0, stream>>>(C, Hit, Linear, Guide, width, height);
-  shadow_species_kernel<<<pool_grid(width, height), kBlock, kBatchSmem, stream>>>(P, Nodes, Order, C, world_trig(), Guide, Linear, width, height, map);
+  if (!batch_smem_ready((const void*)shadow_species_kernel)) return smem_error(name);
+  const TightScratch t(P, Order, Nodes, n_species, C, true, stream);
+  if (t.status) return t.status;
+  shadow_species_kernel<<<pool_grid(width, height), kBlock, t.boxes ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), t.boxes, n_species, Hit, Guide,
+                                                                                  Linear, width, height, map);
   shade_compose_species_kernel<<<pixel_grid(width, height), kBlock, 0, stream>>>(P, C, world_trig(), Hit, Linear, Guide, width, height, map);
-  count_launch(3);
+  count_launch(2);
   return check_launch(name);
 }
 

@@ -2,7 +2,7 @@
 // block prologue shared by the trace/shade kernels and the work-counting
 // kernel.
 #pragma once
-#include "warpbatch.cuh"
+#include "blockbatch.cuh"
 
 namespace arbor {
 namespace {

@@ -1,0 +1,261 @@
+// tight.cuh - tight bounds over the reference's heap BVH, for the batched
+// traversal.
+//
+// A leaf record's bounding box in Nodes (boundLow/boundHigh, Arbor.cu:132-133)
+// is the cube of the leaf's whole reach around its stem base.  The leaf itself
+// (blade box and petiole) fills a small part of it: on the 1080p forest walk a
+// shadow segment tests 547 boxes and 61 leaves to find 5.5 blade boxes.  The
+// trace and shade passes therefore traverse a second set of boxes over the
+// same heap: leaf records bounded by their oriented blade box, inner nodes by
+// the union of their children, everything else as in Nodes.  The boxes are
+// made from P, Order and Nodes by one small kernel in front of each pass (64
+// CTAs per scene, about 6 MB of traffic) and kept nowhere.
+//
+// Why no result changes.  A primitive counts only when the ray passes its box
+// in Nodes, and that test is still made, exactly, on every candidate
+// (batch_tests).  The tight boxes only drop candidates whose test returns no
+// hit.  To be sure of that the traversal widens every tight box by a margin m
+// that covers what the FP32 tests can report off the true surface:
+//  - the sphere and cone quadratics cancel: their discriminant is off by at
+//    most 25 u D^2 (u = 2^-24, D the largest distance from the ray's origin
+//    to the tree's box), so a ray that passes a surface within sqrt(25 u) D =
+//    1.22e-3 D may be reported to hit it, at a t off by as much.  kTightRel =
+//    1.3e-3.
+//  - wind turns a leaf about its blade's cross axis by at most 0.155 wind
+//    radians (load_leaf), which moves a point of it by at most that times its
+//    distance from the stem base (`reach`).
+// Pruning is by the widened box's entry, which no reported t can precede.
+//
+// The boxes are stored 16 bits a coordinate, on a grid over the root's box and
+// rounded outward: the four nodes 4g .. 4g + 3 that a traversal step tests
+// together are 48 bytes (128 in Nodes), three 16-byte loads a lane.  The loads
+// of a step are scattered, one line a lane, and what bounds them is the number
+// of load instructions times lanes; the smaller set also stays in what the
+// passes leave of L1 (28 KB).
+//
+// The boxes are used only where Nodes is what buildBounds makes of P and
+// Order (every leaf box equal to the record's, every inner node the union of
+// its children).  What a scene whose Nodes say anything else shows depends on
+// the order of the traversal; it is traced one tree at a time in a fixed order
+// (tree_in_order).
+#pragma once
+#include "arbor_scene.cuh"
+
+namespace arbor {
+
+constexpr int kTightParts = 64;                          // CTAs per scene; part k owns the subtree of node 64 + k
+constexpr int kTightLeaves = kCapacity / kTightParts;    // 512 leaves each; nodes above the parts keep their box
+constexpr int kTightReach = kNodeCount * 3;              // per part its reach (-1: use Nodes), after the nodes' 3 words each
+constexpr int kTightGrid = kTightReach + kTightParts;    // the grid's origin and step (x, y, z each)
+constexpr int kTightWords = kTightGrid + 8;              // words per scene
+constexpr size_t kTightBytes = sizeof(uint32_t) * kTightWords;
+static_assert(kTightWords % 4 == 0, "16-byte aligned groups in every scene");
+constexpr float kTightRel = 1.3e-3f;
+constexpr float kSwing = 0.156f;  // wind's largest turn per unit (0.11 + 0.045 radians, rounded up)
+
+struct TightPart {
+  float4 lo[kTightLeaves], hi[kTightLeaves];
+};
+
+// Leaf record of one Order slot (Arbor.cu:141): {boundLow, active, boundHigh,
+// id}.  An id outside the 32768 records (invalid input) is given the bounds
+// of an unused record instead of reading out of bounds.
+__device__ __forceinline__ void leaf_record(const float* P, uint32_t uid, float4& lo4, float4& hi4) {
+  if (uid >= (uint32_t)kCapacity) {
+    lo4 = make_float4(kFar, kFar, kFar, 0.0f);
+    hi4 = make_float4(-kFar, -kFar, -kFar, (float)(int)uid);
+    return;
+  }
+  int id = (int)uid;
+  float4 r0 = ldg4(P, id * 6), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2), r4 = ldg4(P, id * 6 + 4);
+  f3 lo, hi;
+  prim_bounds(r0, r1, r1.w, r2.w, r4.x, lo, hi);
+  lo4 = make_float4(lo.x, lo.y, lo.z, r0.w >= 0.0f ? 1.0f : 0.0f);
+  hi4 = make_float4(hi.x, hi.y, hi.z, (float)id);
+}
+// Parent = union of the two children (Arbor.cu:142).
+__device__ __forceinline__ void merge(float4 alo, float4 ahi, float4 clo, float4 chi, float4& plo, float4& phi) {
+  plo = make_float4(fminf(alo.x, clo.x), fminf(alo.y, clo.y), fminf(alo.z, clo.z), alo.w + clo.w);
+  phi = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), -1.0f);
+}
+__device__ __forceinline__ bool same_box(float4 alo, float4 ahi, float4 blo, float4 bhi) {
+  return alo.x == blo.x && alo.y == blo.y && alo.z == blo.z && alo.w == blo.w && ahi.x == bhi.x && ahi.y == bhi.y && ahi.z == bhi.z;
+}
+
+// Interval [a, b] times component c of an axis.
+__device__ __forceinline__ void add_axis(float c, float a, float b, float& lo, float& hi) {
+  lo += fminf(a * c, b * c);
+  hi += fmaxf(a * c, b * c);
+}
+// Shrinks the box (lo, hi) of leaf record `id` to its blade box and petiole
+// in still air and returns the leaf's reach (0: left as it was, the frame is
+// not orthonormal or a size is negative or not finite).
+__device__ __forceinline__ float tighten_leaf(const float* P, int id, float4& lo, float4& hi) {
+  const float4 r0 = ldg4(P, id * 6), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2), r3 = ldg4(P, id * 6 + 3), r4 = ldg4(P, id * 6 + 4);
+  const f3 o = xyz(r0), u = xyz(r1), v = xyz(r2), n = xyz(r3);
+  const float len = r1.w, width = r2.w, stem = r4.x;
+  const float g = fmaxf(fmaxf(fabsf(dot3(u, u) - 1.0f), fmaxf(fabsf(dot3(v, v) - 1.0f), fabsf(dot3(n, n) - 1.0f))),
+                        fmaxf(fabsf(dot3(u, v)), fmaxf(fabsf(dot3(u, n)), fabsf(dot3(v, n)))));
+  const float x1 = stem + len + 0.002f, w = fmaxf(width, 0.002f) + 0.0005f;
+  const float reach = sqrtf(x1 * x1 + w * w + 0.0045f);  // 0.067^2 across
+  if (!(g < 1.0e-4f) || !(len >= 0.0f) || !(stem >= 0.0f) || !(width >= 0.0f) || !(reach < 1.0e3f)) return 0.0f;
+  const float oc[3] = {o.x, o.y, o.z}, uc[3] = {u.x, u.y, u.z}, vc[3] = {v.x, v.y, v.z}, nc[3] = {n.x, n.y, n.z};
+  float l[3], h[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const float slack = 1.0e-3f * reach + 1.0e-6f * fabsf(oc[k]);
+    l[k] = oc[k] - slack;
+    h[k] = oc[k] + slack;
+    add_axis(uc[k], -0.002f, x1, l[k], h[k]);       // blade -0.001 .. len + 0.001 past the stem, petiole radius 0.0011
+    add_axis(vc[k], -w, w, l[k], h[k]);
+    add_axis(nc[k], -0.037f, 0.067f, l[k], h[k]);   // blade box -0.035 .. 0.065 (leaf_clip)
+  }
+  const f3 tl = max3(mk(l[0], l[1], l[2]), xyz(lo)), th = min3(mk(h[0], h[1], h[2]), xyz(hi));
+  if (!(tl.x <= th.x) || !(tl.y <= th.y) || !(tl.z <= th.z)) return 0.0f;
+  lo.x = tl.x, lo.y = tl.y, lo.z = tl.z;
+  hi.x = th.x, hi.y = th.y, hi.z = th.z;
+  return reach;
+}
+
+// The grid of a scene's stored boxes, over its root box: origin and step.
+struct TightGridC {
+  f3 origin, step;
+};
+__device__ __forceinline__ TightGridC tight_grid(const float* Nodes) {
+  const f3 lo = xyz(ldg4(Nodes, 2)), hi = xyz(ldg4(Nodes, 3));
+  return {lo, (hi - lo) * (1.00001f / 65535.0f)};
+}
+__device__ __forceinline__ uint32_t grid_pair(float lo, float hi, float origin, float step) {
+  const float a = fminf(fmaxf(floorf((lo - origin) / step) - 1.0f, 0.0f), 65535.0f);
+  const float b = fminf(fmaxf(ceilf((hi - origin) / step) + 1.0f, 0.0f), 65535.0f);
+  return (uint32_t)a | ((uint32_t)b << 16);
+}
+// Node `node`'s box on the grid: per axis lo | hi << 16.  A box without
+// primitives is stored inside out (lo 65535, hi 0).
+__device__ __forceinline__ void store_tight(uint32_t* T, int node, const TightGridC& g, float4 lo, float4 hi) {
+  uint32_t* t = T + 3 * node;
+  const bool some = lo.w > 0.0f;
+  t[0] = some ? grid_pair(lo.x, hi.x, g.origin.x, g.step.x) : 65535u;
+  t[1] = some ? grid_pair(lo.y, hi.y, g.origin.y, g.step.y) : 65535u;
+  t[2] = some ? grid_pair(lo.z, hi.z, g.origin.z, g.step.z) : 65535u;
+}
+
+// Part `part` of a scene's tight boxes, by one CTA of 256 threads.
+__device__ __forceinline__ void tight_build_part(TightPart& s, const float* __restrict__ P, const uint32_t* __restrict__ Order,
+                                                 const float* __restrict__ Nodes, uint32_t* __restrict__ T, int part) {
+  const int tid = threadIdx.x;
+  const TightGridC g = tight_grid(Nodes);
+  // (a grid that is not finite, or has no extent on an axis, holds nothing)
+  bool bad = !(g.step.x > 1.0e-20f && g.step.y > 1.0e-20f && g.step.z > 1.0e-20f && fmaxf(g.step.x, fmaxf(g.step.y, g.step.z)) < 1.0f);
+  float reach = 0.0f;
+  for (int k = tid; k < kTightLeaves; k += blockDim.x) {
+    const int slot = part * kTightLeaves + k, node = kCapacity + slot;
+    const uint32_t uid = __ldg(Order + slot);
+    const float4 nlo = ldg4(Nodes, 2 * node), nhi = ldg4(Nodes, 2 * node + 1);
+    float4 lo, hi;
+    leaf_record(P, uid, lo, hi);
+    bad |= !same_box(lo, hi, nlo, nhi);
+    if (uid < (uint32_t)kCapacity && (int)ldg4(P, (int)uid * 6).w == 1) reach = fmaxf(reach, tighten_leaf(P, (int)uid, lo, hi));
+    s.lo[k] = lo;
+    s.hi[k] = hi;
+    store_tight(T, node, g, lo, hi);
+  }
+  // Nodes' inner nodes: the unions of their children?  (part 0 also looks at
+  // the nodes above the parts)
+  for (int k = tid; k < kTightLeaves; k += blockDim.x) {
+    if (k > 0) {  // the k-th inner node of this part's subtree, k = 1 its root
+      const int depth = 31 - __clz(k);
+      const int node = ((kTightParts + part) << depth) + (k - (1 << depth));
+      float4 plo, phi;
+      merge(ldg4(Nodes, 4 * node), ldg4(Nodes, 4 * node + 1), ldg4(Nodes, 4 * node + 2), ldg4(Nodes, 4 * node + 3), plo, phi);
+      bad |= !same_box(plo, phi, ldg4(Nodes, 2 * node), ldg4(Nodes, 2 * node + 1));
+    }
+  }
+  if (part == 0 && tid < kTightParts) {
+    const float4 lo = ldg4(Nodes, 2 * tid), hi = ldg4(Nodes, 2 * tid + 1);
+    store_tight(T, tid, g, tid > 1 ? lo : make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi);  // 0 and 1 are no one's children: empty
+    if (tid > 0) {
+      float4 plo, phi;
+      merge(ldg4(Nodes, 4 * tid), ldg4(Nodes, 4 * tid + 1), ldg4(Nodes, 4 * tid + 2), ldg4(Nodes, 4 * tid + 3), plo, phi);
+      bad |= !same_box(plo, phi, lo, hi);
+    }
+  }
+  __syncthreads();
+  int first = kCapacity + part * kTightLeaves;
+  for (int width = kTightLeaves / 2; width >= 1; width >>= 1) {
+    first >>= 1;
+    float4 plo, phi;
+    if (tid < width) merge(s.lo[2 * tid], s.hi[2 * tid], s.lo[2 * tid + 1], s.hi[2 * tid + 1], plo, phi);
+    __syncthreads();
+    if (tid < width) {
+      s.lo[tid] = plo;
+      s.hi[tid] = phi;
+      store_tight(T, first + tid, g, plo, phi);
+    }
+    __syncthreads();
+  }
+  // the part's reach (non-negative floats order as their bits do)
+  __shared__ int part_reach;
+  if (tid == 0) part_reach = 0;
+  const bool any_bad = __syncthreads_or(bad);
+  atomicMax(&part_reach, __float_as_int(reach));
+  __syncthreads();
+  if (tid == 0) T[kTightReach + part] = any_bad ? __float_as_uint(-1.0f) : (uint32_t)part_reach;
+  if (part == 0 && tid == 0) {
+    const float v[6] = {g.origin.x, g.origin.y, g.origin.z, g.step.x, g.step.y, g.step.z};
+    for (int k = 0; k < 6; k++) T[kTightGrid + k] = __float_as_uint(v[k]);
+  }
+}
+static_assert(kTightLeaves / 2 == 256, "one thread per node of the widest inner level");
+
+// What a pass traverses.
+struct TightView {
+  const uint32_t* T;  // the tight boxes of its scene(s), kTightWords each; null: Nodes
+  bool regular;       // Nodes is what buildBounds makes of P and Order
+  float rel, abs;     // the boxes' margin: rel x D + abs
+};
+// Largest swing of a leaf under `wind` whose reach is `reach`.
+__device__ __forceinline__ float swing_margin(float wind, float reach) { return fminf(fabsf(wind) * kSwing, 2.0f) * reach; }
+
+// One warp: the view of one scene's tight boxes.
+__device__ __forceinline__ TightView tight_view_warp(const uint32_t* T, float wind) {
+  const int lane = threadIdx.x & 31;
+  const float a = __uint_as_float(__ldg(T + kTightReach + lane)), b = __uint_as_float(__ldg(T + kTightReach + 32 + lane));
+  if (__any_sync(0xffffffffu, !(a >= 0.0f) || !(b >= 0.0f))) return {nullptr, false, 0.0f, 0.0f};
+  const int reach = __reduce_max_sync(0xffffffffu, __float_as_int(fmaxf(a, b)));
+  return {T, true, kTightRel, swing_margin(wind, __int_as_float(reach))};
+}
+// A block: the view of n scenes' tight boxes; T null: of the scenes
+// themselves, whose Nodes the block then looks through (5 MB a scene; passes
+// without scratch are rare).  Every thread calls it.
+__device__ __forceinline__ TightView tight_view_block(const uint32_t* T, const float* __restrict__ P, const uint32_t* __restrict__ Order,
+                                                      const float* __restrict__ Nodes, int n, float wind) {
+  __shared__ int reach;
+  if (threadIdx.x == 0) reach = 0;
+  __syncthreads();
+  bool bad = false;
+  if (T == nullptr) {
+    for (int s = 0; s < n; s++) {
+      const float* p = P + (size_t)s * (kCapacity * kPS);
+      const float* nodes = Nodes + (size_t)s * (kNodeCount * 8);
+      for (int k = threadIdx.x; k < kCapacity; k += blockDim.x) {
+        float4 lo, hi;
+        leaf_record(p, __ldg(Order + (size_t)s * kCapacity + k), lo, hi);
+        bad |= !same_box(lo, hi, ldg4(nodes, 2 * (kCapacity + k)), ldg4(nodes, 2 * (kCapacity + k) + 1));
+        if (k == 0) continue;
+        merge(ldg4(nodes, 4 * k), ldg4(nodes, 4 * k + 1), ldg4(nodes, 4 * k + 2), ldg4(nodes, 4 * k + 3), lo, hi);
+        bad |= !same_box(lo, hi, ldg4(nodes, 2 * k), ldg4(nodes, 2 * k + 1));
+      }
+    }
+    return {nullptr, !__syncthreads_or(bad), 0.0f, 0.0f};
+  }
+  for (int k = threadIdx.x; k < n * kTightParts; k += blockDim.x) {
+    const float r = __uint_as_float(__ldg(T + (size_t)(k / kTightParts) * kTightWords + kTightReach + k % kTightParts));
+    bad |= !(r >= 0.0f);
+    atomicMax(&reach, __float_as_int(r));
+  }
+  if (__syncthreads_or(bad)) return {nullptr, false, 0.0f, 0.0f};
+  return {T, true, kTightRel, swing_margin(wind, __int_as_float(reach))};
+}
+
+}  // namespace arbor
