@@ -79,6 +79,10 @@ struct ConvArgs {
   // [0, cs) - the decoder's concatenation, read without being stored.
   const bf16* x2;
   int cs;
+  // The output layer in inference (tcgen05): the denoised image (float4 per
+  // pixel) from the base image and the layer's first three channels.
+  const float4* base;
+  float4* denoised;
 };
 
 // Address of input channels [c, c + 8) of pixel (img, gy, gx).
@@ -185,44 +189,54 @@ __global__ void __launch_bounds__(128) conv_kernel(ConvArgs a) {
 }
 
 // ------------------------------------------- tcgen05 convolution (sm_100a) --
-// The same 3x3 convolution on the 5th-generation tensor cores: a CTA of 4
-// warps computes R consecutive output rows of a 128-pixel column segment for
-// all N output channels.  Per chunk of CC input channels it stages the R + 2
-// input rows (130 pixels with the halo) and the chunk's weights in shared
-// memory with cp.async (two stage buffers: chunk c + 1 loads while chunk c's
-// MMAs run), in the K-major, non-swizzled core-matrix layout the
-// MMA reads (8 rows of 16 bytes per core matrix): the A operand of output row
-// r and tap (dy, dx) is staged row r + dy shifted by dx, so one 128-row
-// descriptor per (row, tap) needs no copy.  One thread issues tcgen05.mma
-// (M = 128, N, K = 16, BF16 inputs, FP32 accumulators in TMEM, one N-column
-// block per output row) for R rows x 9 taps x CC/16 steps and commits to an
-// mbarrier; every thread waits (bounded) for a chunk's MMAs before its stage
-// buffer is refilled.  The epilogue reads the accumulators with tcgen05.ld (warp w owns
-// TMEM lanes 32w..32w+31 = pixels 32w..32w+31 of the segment), applies bias
-// and activation and stores BF16 or FP32.
+// The same 3x3 convolution on the 5th-generation tensor cores, in two forms of
+// one warp-specialised pipeline.  A CTA works on a 128-pixel column segment:
+// four producer warps copy input rows (130 pixels with the halo) and weights
+// into shared memory with cp.async, in the K-major, non-swizzled core-matrix
+// layout the MMA reads (8 rows of 16 bytes per core matrix), so that the A
+// operand of an output row and a tap (dy, dx) is a staged row shifted by dx and
+// needs no copy; one thread issues tcgen05.mma (M = 128, N, K = 16, BF16
+// inputs, FP32 accumulators in TMEM); four epilogue warps read finished
+// accumulators with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = pixels
+// 32w..32w+31 of the segment), apply bias and activation and store.  The roles
+// meet on mbarriers only: the copies run as far ahead as the ring of stages
+// allows, the MMAs of a row run while earlier rows are stored.  (With all
+// threads copying, waiting and storing in turn, one row ahead, a 32 -> 32 row
+// took 6,500 cycles for 576 cycles of MMAs: the time was the latency of one
+// copy after another.)
+//
+// Waits are bounded: a role that gives up sets the CTA's fail flag and the
+// error word, every other role sees the flag in its own waits, and the CTA
+// ends with its copies done and its TMEM freed.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   // start address, leading / stride byte offsets (16-byte units), version 1,
   // no swizzle (layout type 0)
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) |
          (1ull << 46);
 }
-template <int N>
-constexpr uint32_t umma_idesc() {
+constexpr __host__ __device__ uint32_t umma_idesc(int N) {
   // FP32 accumulator, BF16 A and B, both K-major, N >> 3, M = 128 >> 4
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 constexpr int pow2_cols(int c) { return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : c <= 256 ? 256 : 512; }
-template <int N, int CC, int R>
-constexpr int conv_tc_stage_bytes() {
-  return (CC / 8) * (R + 2) * 130 * 16 + 9 * (CC / 8) * N * 16;
+__device__ __forceinline__ void umma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(da), "l"(db), "r"(idesc), "r"(accumulate ? 1u : 0u));
 }
-template <int N, int CC, int R>
-constexpr int conv_tc_smem_bytes() {
-  return 2 * conv_tc_stage_bytes<N, CC, R>() + N * 4 + 16;  // two stages, biases, mbarrier, TMEM slot
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
-
-// Bounded wait on an mbarrier phase; false when it did not complete.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
+__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(bar) : "memory");
+}
+// Bounded wait on an mbarrier phase; false when it did not complete or another
+// role has given up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, const volatile int* fail) {
   for (int i = 0; i < (1 << 20); i++) {
     uint32_t done;
     asm volatile(
@@ -231,6 +245,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
         : "r"(bar), "r"(phase)
         : "memory");
     if (done) return true;
+    if (*fail) return false;
   }
   return false;
 }
@@ -238,316 +253,403 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
   // a 16-byte copy, or 16 zero bytes when !valid (src-size 0)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int K>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-template <int N, int CC, int R>
-__global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs a, int* err) {
-  extern __shared__ __align__(128) uint8_t tc_smem[];
-  constexpr int KU = CC / 8;                    // 16-byte K units per chunk
-  constexpr int ROWS = R + 2;                   // staged input rows
-  constexpr int HALO_B = KU * ROWS * 130 * 16;
-  constexpr int STAGE_B = conv_tc_stage_bytes<N, CC, R>();
-  constexpr uint32_t LBO_A = ROWS * 130 * 16;   // next K unit of the staged rows
-  constexpr uint32_t LBO_B = N * 16;            // next K unit of the weights
-  constexpr int COLS = pow2_cols(R * N);
-  float* bias_s = reinterpret_cast<float*>(tc_smem + 2 * STAGE_B);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(bias_s + N);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_x = (a.w + 127) >> 7, rows_y = (a.h + R - 1) / R;
-  int t = blockIdx.x;
-  const int tx = t % tiles_x;
-  t /= tiles_x;
-  const int y0 = (t % rows_y) * R, img = t / rows_y;
-  const int x0 = tx * 128;
-  const uint32_t bar_a = smem_u32(bar);
-  const uint32_t smem_a = smem_u32(tc_smem);
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(COLS));
+constexpr int kProducers = 256;
+constexpr int kMmaWarp = 4 + kProducers / 32;          // epilogue warps 0-3, producer warps, MMA warp
+constexpr int kConvThreads = (kMmaWarp + 1) * 32;
+
+// One pixel's 16 output channels from col: bias, activation or activation
+// derivative, store (32 bytes of BF16, or 64 of FP32).
+__device__ __forceinline__ void conv_store16(const ConvArgs& a, size_t p, int col, const uint32_t* v, const float* bias_s) {
+  float f[16];
+  uint4 m[2];
+  if (a.mask) {
+    const uint4* mp = reinterpret_cast<const uint4*>(a.mask + p * a.cout + col);
+    m[0] = __ldg(mp);
+    m[1] = __ldg(mp + 1);
+  }
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    float x = __uint_as_float(v[j]) + bias_s[col + j];
+    if (a.act) x = x > 0.0f ? x : x * kSlope;
+    if (a.mask && !(__bfloat162float(reinterpret_cast<const bf16*>(m)[j]) > 0.0f)) x *= kSlope;
+    f[j] = x;
+  }
+  if (a.denoised) {  // the output layer in inference: log(1 + base) + out[0:3], back to radiance
+    const float4 nz = __ldg(a.base + p);
+    a.denoised[p] = make_float4(expm1f(log1pf(fmaxf(nz.x, 0.0f)) + f[0]), expm1f(log1pf(fmaxf(nz.y, 0.0f)) + f[1]),
+                                expm1f(log1pf(fmaxf(nz.z, 0.0f)) + f[2]), 1.0f);
+  } else if (a.y_fp32) {
+    float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.y) + p * a.cout + col);
+#pragma unroll
+    for (int j = 0; j < 4; j++) o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+  } else {
+    uint32_t w[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+      w[j] = *reinterpret_cast<const uint32_t*>(&b2);
+    }
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(reinterpret_cast<bf16*>(a.y) + p * a.cout + col), "r"(w[0]), "r"(w[1]),
+                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+        "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
+}
+// One accumulator row (N columns from tmem address t, this warp's lanes) of
+// pixel p; `live`: the pixel is inside the image.
+template <int N>
+__device__ __forceinline__ void conv_epilogue_row(const ConvArgs& a, uint32_t t, size_t p, bool live, const float* bias_s) {
+#pragma unroll
+  for (int col = 0; col < N; col += 32) {
+    constexpr int W = N < 32 ? 16 : 32;
+    uint32_t v[W];
+#pragma unroll
+    for (int k = 0; k < W; k += 16) tmem_ld16(t + (uint32_t)(col + k), v + k);
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+    if (live)
+#pragma unroll
+      for (int k = 0; k < W; k += 16) conv_store16(a, p, col + k, v + k, bias_s);
+  }
+}
+
+// Copies input row gy's units of channels [c0, c0 + 8 KU) of the segment at x0
+// to dst, unit (k, hx) at k * kstride + hx * 16.  A thread copies one k of
+// every (T / KU)-th pixel, so that its addresses advance by constants.
+constexpr int kUnitPitch = 136 * 16;  // 130 pixels of 16 bytes, to whole 128-byte lines
+template <int KU>
+__device__ __forceinline__ void conv_stage_row(const ConvArgs& a, int img, int gy, int x0, int c0, uint32_t dst, uint32_t kstride, int ptid) {
+  constexpr int T = kProducers / KU * KU, STEP = T / KU;
+  if (ptid >= T) return;
+  const int k = ptid % KU, h0 = ptid / KU, c = c0 + k * 8;
+  const bool row_in = gy >= 0 && gy < a.h;
+  const int c1 = a.x2 ? a.cs : a.cin;  // channels of a pixel of x
+  dst += k * kstride + h0 * 16;
+  int gx = x0 + h0 - 1;
+  if (c < c1) {
+    const bf16* src = a.x + ((size_t)(img * a.h + (row_in ? gy : 0)) * a.w) * c1 + c;
+    for (int hx = h0; hx < 130; hx += STEP, gx += STEP, dst += STEP * 16) {
+      const bool in = row_in && gx >= 0 && gx < a.w;
+      cp_async16(dst, in ? src + (size_t)(gx * c1) : a.x, in);
+    }
+  } else {
+    const int c2 = a.cin - a.cs;
+    const bf16* src = a.x2 + ((size_t)(img * (a.h >> 1) + (row_in ? gy >> 1 : 0)) * (a.w >> 1)) * c2 + (c - a.cs);
+    for (int hx = h0; hx < 130; hx += STEP, gx += STEP, dst += STEP * 16) {
+      const bool in = row_in && gx >= 0 && gx < a.w;
+      cp_async16(dst, in ? src + (size_t)((gx >> 1) * c2) : a.x, in);
+    }
+  }
+}
+// Copies the weights of input channels [c0, c0 + 8 KU): unit (dx, k, j, n) at
+// (((dx * KU + k) * 3 + j) * N + n) * 16, j = 2 - dy.
+template <int N, int KU>
+__device__ __forceinline__ void conv_stage_weights(const ConvArgs& a, int c0, uint32_t dst, int ptid) {
+  for (int v = ptid; v < 9 * KU * N; v += kProducers) {
+    const int k = v % KU, q = v / KU;
+    const int tap = q % 9, n = q / 9;
+    const int dy = tap / 3, dx = tap - 3 * dy;
+    const bool in = n < a.cout;
+    cp_async16(dst + (((dx * KU + k) * 3 + 2 - dy) * N + n) * 16, in ? a.wt + ((size_t)n * 9 + tap) * a.cin + c0 + k * 8 : a.wt, in);
+  }
+}
+// The MMAs of one 16-channel step (A descriptor da) of one tap column on the
+// accumulators of COUNT successive output rows at tmem columns acc: weights
+// db of the first row's dy, the other rows' behind them.  At most 256 columns
+// at a time.  (One thread issues them all: counts are compile-time constants,
+// a loop over them took as long as the MMAs.)
+template <int N, int COUNT>
+__device__ __forceinline__ void umma_rows(uint32_t acc, uint64_t da, uint64_t db, bool accumulate) {
+  constexpr int MAX = 256 / N;
+#pragma unroll
+  for (int k = 0; k < COUNT; k += MAX)
+    umma(acc + (uint32_t)(k * N), da, db + (uint64_t)(k * N), umma_idesc((COUNT - k < MAX ? COUNT - k : MAX) * N), accumulate);
+}
+template <int N>
+__device__ __forceinline__ void umma_rows_of(int count, uint32_t acc, uint64_t da, uint64_t db, bool accumulate) {
+  if (count == 1) umma_rows<N, 1>(acc, da, db, accumulate);
+  if (count == 2) umma_rows<N, 2>(acc, da, db, accumulate);
+  if (count == 3) umma_rows<N, 3>(acc, da, db, accumulate);
+}
+
+// Shared-memory control block of a pipeline of S stages and B accumulators.
+template <int S, int B>
+struct ConvCtl {
+  uint64_t full[S], empty[S], acc_full[B], acc_empty[B];
+  uint32_t tmem;
+  int fail;
+};
+template <int S, int B>
+__device__ __forceinline__ void conv_ctl_init(ConvCtl<S, B>& c, int cols) {
+  const int tid = threadIdx.x;
+  if (tid >> 5 == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&c.tmem)), "r"(cols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar_a), "r"(1));
+    for (int k = 0; k < S; k++) {
+      mbar_init(smem_u32(&c.full[k]), kProducers);
+      mbar_init(smem_u32(&c.empty[k]), 1);
+    }
+    for (int k = 0; k < B; k++) {
+      mbar_init(smem_u32(&c.acc_full[k]), 1);
+      mbar_init(smem_u32(&c.acc_empty[k]), 128);
+    }
+    c.fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
   }
-  for (int i = tid; i < N; i += 128) bias_s[i] = a.bias && i < a.cout ? a.bias[i] : 0.0f;
-  // Stage the operands of the chunk starting at channel c0 into stage buffer sb.
-  auto stage = [&](int c0, int sb) {
-    const uint32_t halo_a = smem_a + sb * STAGE_B, wts_a = halo_a + HALO_B;
-    for (int v = tid; v < ROWS * 130 * KU; v += 128) {
-      const int k = v % KU, rh = v / KU;
-      const int r = rh / 130, hx = rh - r * 130;
-      const int gy = y0 + r - 1, gx = x0 + hx - 1;
-      const bool in = gy >= 0 && gy < a.h && gx >= 0 && gx < a.w;
-      const bf16* src = in ? conv_in(a.x, a.x2, a.cin, a.cs, a.h, a.w, img, gy, gx, c0 + k * 8) : a.x;
-      cp_async16(halo_a + ((k * ROWS + r) * 130 + hx) * 16, src, in);
-    }
-    for (int v = tid; v < 9 * KU * N; v += 128) {
-      const int k = v % KU, q = v / KU;
-      const int tap = q % 9, n = q / 9;
-      const bool in = n < a.cout;
-      const bf16* src = in ? a.wt + ((size_t)n * 9 + tap) * a.cin + c0 + k * 8 : a.wt;
-      cp_async16(wts_a + ((tap * KU + k) * N + n) * 16, src, in);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-  const uint32_t tmem = *tmem_slot;
-  const int chunks = a.cin / CC;
-  bool ok = true;
-  stage(0, 0);
-  for (int c = 0; c < chunks && ok; c++) {
-    // The chunk c-1 MMAs must be done before their buffer takes chunk c+1.
-    if (c > 0) ok = __syncthreads_and(mbar_wait(bar_a, (uint32_t)((c - 1) & 1)) ? 1 : 0) != 0;
-    if (!ok) break;
-    if (c + 1 < chunks) {
-      stage((c + 1) * CC, (c + 1) & 1);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // chunk c's copies are in
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-    // make the staged operands visible to the tensor cores
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-      const uint32_t idesc = umma_idesc<N>();
-      const uint32_t halo_a = smem_a + (c & 1) * STAGE_B, wts_a = halo_a + HALO_B;
-      // descriptors advance by address only (16-byte units in the low bits)
-      const uint64_t da0 = umma_desc(halo_a, LBO_A, 128), db0 = umma_desc(wts_a, LBO_B, 128);
-      uint32_t acc = c > 0 ? 1u : 0u;
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-#pragma unroll
-        for (int tap = 0; tap < 9; tap++) {
-#pragma unroll
-          for (int st = 0; st < CC / 16; st++) {
-            const uint64_t da = da0 + (uint64_t)((((2 * st * ROWS + r + tap / 3) * 130 + tap % 3) * 16) >> 4);
-            const uint64_t db = db0 + (uint64_t)(((tap * KU + 2 * st) * N * 16) >> 4);
-            const uint32_t acc_rt = (tap > 0 || st > 0) ? 1u : acc;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + (uint32_t)(r * N)),
-                "l"(da), "l"(db), "r"(idesc), "r"(acc_rt));
-          }
-        }
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar_a) : "memory");
-    }
-  }
-  // the last chunk's MMAs (bounded, uniform outcome)
-  if (ok) ok = __syncthreads_and(mbar_wait(bar_a, (uint32_t)((chunks - 1) & 1)) ? 1 : 0) != 0;
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+template <int S, int B>
+__device__ __forceinline__ void conv_ctl_end(ConvCtl<S, B>& c, int cols, bool ok, int* err) {
   if (!ok) {
-    if (tid == 0) atomicExch(err, 1);
-  } else {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-    const int gx = x0 + warp * 32 + lane;  // this thread's TMEM lane = pixel of the segment
-#pragma unroll 1
-    for (int r = 0; r < R; r++) {
-      const int gy = y0 + r;
-      const size_t p = (size_t)(img * a.h + gy) * a.w + gx;
-#pragma unroll 1
-      for (int col = 0; col < N; col += 16) {
-        uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-              "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(r * N + col)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (gx < a.w && gy < a.h) {
-          float f[16];
-#pragma unroll
-          for (int j = 0; j < 16; j++) {
-            const int co = col + j;
-            float x = __uint_as_float(v[j]) + bias_s[co];
-            if (a.act) x = x > 0.0f ? x : x * kSlope;
-            if (a.mask && !(__bfloat162float(a.mask[p * a.cout + co]) > 0.0f)) x *= kSlope;
-            f[j] = x;
-          }
-          if (a.y_fp32) {
-            float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.y) + p * a.cout + col);
-#pragma unroll
-            for (int j = 0; j < 4; j++) o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-          } else {
-            uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(a.y) + p * a.cout + col);
-            uint32_t w[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-              const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-              w[j] = *reinterpret_cast<const uint32_t*>(&b2);
-            }
-            o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            o[1] = make_uint4(w[4], w[5], w[6], w[7]);
-          }
-        }
-      }
-    }
+    *reinterpret_cast<volatile int*>(&c.fail) = 1;
+    atomicExch(err, 1);
   }
+  cp_wait<0>();
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(COLS));
+  if (threadIdx.x >> 5 == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(c.tmem), "r"(cols));
 }
 
-// Row-streaming form for the layers whose weights fit in shared memory
-// with a 5-row input ring: a CTA keeps all 9 x CIN x N weights resident and
-// walks down its rows of one 128-pixel column segment.  Per output row y it
-// starts loading input row y + 2 (all CIN channels, cp.async) into the ring,
-// waits for row y + 1, one thread issues the row's 9 x CIN/16 MMAs into one
-// of two TMEM accumulators, and the 4 warps run the previous row's epilogue
-// while those MMAs execute; each input row is read from memory once per
-// segment.
-template <int N, int CIN>
+// Row-streaming form, for the layers whose weights fit in shared memory beside
+// a ring of S input rows: a CTA keeps all 9 x CIN x N weights resident and
+// walks down rows_per_cta rows of its segment; each input row is read once per
+// segment, up to S rows ahead of the MMAs.
+//
+// An input row feeds three output rows, one per dy.  Their accumulators are
+// neighbours in TMEM (a ring of B blocks of N columns) and the three dy's
+// weights neighbours in shared memory, so one MMA of 3 N columns does all
+// three: what an MMA costs here is reading its A operand (128 pixels x 16
+// channels: measured 150-200 cycles for N = 32 .. 96), and a row's A is read 3
+// times, once per dx, instead of 9.  The products of an output still come in
+// the order dy, dx, channel step.
+template <int N, int CIN, int S, int B>
 constexpr int conv_row_smem_bytes() {
-  return 9 * (CIN / 8) * N * 16 + 5 * (CIN / 8) * 130 * 16 + N * 4 + 32;
+  return 9 * (CIN / 8) * N * 16 + S * (CIN / 8) * kUnitPitch + N * 4 + (int)sizeof(ConvCtl<S, B>) + 16;
 }
-
-template <int N, int CIN>
-__global__ void __launch_bounds__(128) conv_row_kernel(ConvArgs a, int rows_per_cta, int* err) {
+template <int N, int CIN, int S, int B>
+__global__ void __launch_bounds__(kConvThreads) conv_row_kernel(const ConvArgs a, int rows_per_cta, int* err) {
   extern __shared__ __align__(128) uint8_t rs_smem[];
-  constexpr int KU = CIN / 8;
+  constexpr int KU = CIN / 8, KS = CIN / 16;
   constexpr int W_B = 9 * KU * N * 16;
-  constexpr int SLOT_B = KU * 130 * 16;        // one staged input row
-  constexpr uint32_t LBO_A = 130 * 16;         // next K unit within a staged row
-  constexpr uint32_t LBO_B = N * 16;           // next K unit of the weights
-  constexpr int COLS = pow2_cols(2 * N);
-  const uint32_t smem_a = smem_u32(rs_smem);
-  const uint32_t wts_a = smem_a, ring_a = smem_a + W_B;
-  float* bias_s = reinterpret_cast<float*>(rs_smem + W_B + 5 * SLOT_B);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(bias_s + N);  // two mbarriers, one per accumulator
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 2);
+  constexpr int SLOT_B = KU * kUnitPitch;      // one staged input row
+  constexpr uint32_t LBO_B = 3 * N * 16;       // next K unit of the weights
+  constexpr int COLS = pow2_cols(B * N);
+  constexpr int L = S - 1;                     // rows in flight
+  const uint32_t wts_a = smem_u32(rs_smem), ring_a = wts_a + W_B;
+  ConvCtl<S, B>& ctl = *reinterpret_cast<ConvCtl<S, B>*>(rs_smem + W_B + S * SLOT_B);
+  float* bias_s = reinterpret_cast<float*>(rs_smem + W_B + S * SLOT_B + (sizeof(ConvCtl<S, B>) + 15) / 16 * 16);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tiles_x = (a.w + 127) >> 7, groups = (a.h + rows_per_cta - 1) / rows_per_cta;
   int t = blockIdx.x;
   const int tx = t % tiles_x;
   t /= tiles_x;
   const int y_begin = (t % groups) * rows_per_cta, img = t / groups;
-  const int y_end = y_begin + rows_per_cta < a.h ? y_begin + rows_per_cta : a.h;
+  const int rows = min(rows_per_cta, a.h - y_begin);  // output rows; input row i is image row y_begin - 1 + i
   const int x0 = tx * 128;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(1));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar + 1)), "r"(1));
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
-  }
-  for (int i = tid; i < N; i += 128) bias_s[i] = a.bias && i < a.cout ? a.bias[i] : 0.0f;
-  // weights: unit (tap, k, n)
-  for (int v = tid; v < 9 * KU * N; v += 128) {
-    const int k = v % KU, q = v / KU;
-    const int tap = q % 9, n = q / 9;
-    const bool in = n < a.cout;
-    cp_async16(wts_a + ((tap * KU + k) * N + n) * 16, in ? a.wt + ((size_t)n * 9 + tap) * a.cin + k * 8 : a.wt, in);
-  }
-  // input row gy into its ring slot (gy + 5) % 5: unit (k, hx)
-  auto load_row = [&](int gy) {
-    const uint32_t slot = ring_a + ((gy + 5) % 5) * SLOT_B;
-    for (int v = tid; v < 130 * KU; v += 128) {
-      const int k = v % KU, hx = v / KU;
-      const int gx = x0 + hx - 1;
-      const bool in = gy >= 0 && gy < a.h && gx >= 0 && gx < a.w;
-      const bf16* src = in ? conv_in(a.x, a.x2, a.cin, a.cs, a.h, a.w, img, gy, gx, k * 8) : a.x;
-      cp_async16(slot + (k * 130 + hx) * 16, src, in);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  load_row(y_begin - 1);
-  load_row(y_begin);
-  load_row(y_begin + 1);
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = umma_idesc<N>();
+  for (int i = tid; i < N; i += kConvThreads) bias_s[i] = a.bias && i < a.cout ? a.bias[i] : 0.0f;
+  conv_ctl_init(ctl, COLS);
+  const volatile int* fail = &ctl.fail;
+  const uint32_t tmem = ctl.tmem;
   bool ok = true;
-  // epilogue of output row y from accumulator (y - y_begin) & 1
-  auto epilogue = [&](int y) {
-    const int b = (y - y_begin) & 1;
-    const bool done = mbar_wait(smem_u32(bar + b), (uint32_t)(((y - y_begin) >> 1) & 1));
-    ok = __syncthreads_and(done ? 1 : 0) != 0;
-    if (!ok) return;
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-    const int gx = x0 + warp * 32 + lane;
-    const size_t p = (size_t)(img * a.h + y) * a.w + gx;
-#pragma unroll 1
-    for (int col = 0; col < N; col += 16) {
-      uint32_t v[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-            "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * N + col)));
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-      if (gx < a.w) {
-        float f[16];
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-          float x = __uint_as_float(v[j]) + bias_s[col + j];
-          if (a.act) x = x > 0.0f ? x : x * kSlope;
-          if (a.mask && !(__bfloat162float(a.mask[p * a.cout + col + j]) > 0.0f)) x *= kSlope;
-          f[j] = x;
-        }
-        if (a.y_fp32) {
-          float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.y) + p * a.cout + col);
-#pragma unroll
-          for (int j = 0; j < 4; j++) o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-        } else {
-          uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(a.y) + p * a.cout + col);
-          uint32_t w[8];
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-            w[j] = *reinterpret_cast<const uint32_t*>(&b2);
-          }
-          o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-          o[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
+  if (warp >= 4 && warp < kMmaWarp) {
+    const int ptid = tid - 128;
+    conv_stage_weights<N, KU>(a, 0, wts_a, ptid);  // complete with the first row
+    for (int i = 0; i < rows + 2 && ok; i++) {
+      if (i >= S) ok = mbar_wait(smem_u32(&ctl.empty[i % S]), (uint32_t)((i / S - 1) & 1), fail);
+      if (!ok) break;
+      conv_stage_row<KU>(a, img, y_begin - 1 + i, x0, 0, ring_a + (i % S) * SLOT_B, kUnitPitch, ptid);
+      cp_commit();
+      if (i >= L) {
+        cp_wait<L>();
+        fence_async();  // the landed row becomes visible to the tensor cores
+        mbar_arrive(smem_u32(&ctl.full[(i - L) % S]));
       }
     }
-    // the accumulator is read out before its next MMAs are issued
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-  };
-  for (int y = y_begin; y < y_end && ok; y++) {
-    // Row y + 2's slot held row y - 3, last read by output row y - 2, whose
-    // MMAs completed before its epilogue (the previous iteration).
-    load_row(y + 2);
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // rows up to y + 1 are in
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-      const uint32_t acc_t = tmem + (uint32_t)(((y - y_begin) & 1) * N);
+    if (ok) {
+      cp_wait<0>();
+      fence_async();
+      for (int i = max(0, rows + 2 - L); i < rows + 2; i++) mbar_arrive(smem_u32(&ctl.full[i % S]));
+    }
+  } else if (warp == kMmaWarp) {
+    if (lane == 0) {
       const uint64_t db0 = umma_desc(wts_a, LBO_B, 128);
+      for (int i = 0; i < rows + 2 && ok; i++) {
+        // input row i: output rows i - 2 (dy 2), i - 1 (dy 1), i (dy 0: its first)
+        ok = mbar_wait(smem_u32(&ctl.full[i % S]), (uint32_t)((i / S) & 1), fail);
+        if (ok && i >= B && i < rows) ok = mbar_wait(smem_u32(&ctl.acc_empty[i % B]), (uint32_t)((i / B - 1) & 1), fail);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+        const int first = max(0, i - 2), last = min(rows - 1, i);
+        const int head = min(last - first + 1, B - first % B);  // rows before the accumulator ring wraps
+        const uint32_t acc = tmem + (uint32_t)((first % B) * N);
+        const uint64_t da0 = umma_desc(ring_a + (i % S) * SLOT_B, kUnitPitch, 128);
+        const uint64_t db1 = db0 + (uint64_t)((first - (i - 2)) * N);
+        const int count = last - first + 1;
+        if (count == 3 && head == 3) {  // in the middle of the segment and of the ring
 #pragma unroll
-      for (int tap = 0; tap < 9; tap++) {
-        const int dy = tap / 3, dx = tap - dy * 3;
-        const uint64_t da0 = umma_desc(ring_a + ((y - 1 + dy + 5) % 5) * SLOT_B, LBO_A, 128);
-#pragma unroll
-        for (int st = 0; st < CIN / 16; st++) {
-          const uint64_t da = da0 + (uint64_t)(((2 * st * 130 + dx) * 16) >> 4);
-          const uint64_t db = db0 + (uint64_t)(((tap * KU + 2 * st) * N * 16) >> 4);
-          const uint32_t acc = (tap > 0 || st > 0) ? 1u : 0u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(acc_t),
-              "l"(da), "l"(db), "r"(idesc), "r"(acc));
+          for (int q = 0; q < 3 * KS; q++) {
+            const int dx = q / KS, st = q % KS;
+            const uint64_t da = da0 + (uint64_t)((2 * st * kUnitPitch + dx * 16) >> 4);
+            const uint64_t db = db1 + (uint64_t)(((dx * KU + 2 * st) * 3 * N * 16) >> 4);
+            if (q == 0) {  // row i's accumulator starts here
+              umma_rows<N, 2>(acc, da, db, true);
+              umma_rows<N, 1>(acc + 2 * N, da, db + (uint64_t)(2 * N), false);
+            } else {
+              umma_rows<N, 3>(acc, da, db, true);
+            }
+          }
+        } else {
+#pragma unroll 1
+          for (int q = 0; q < 3 * KS; q++) {
+            const int dx = q / KS, st = q % KS;
+            const uint64_t da = da0 + (uint64_t)((2 * st * kUnitPitch + dx * 16) >> 4);
+            const uint64_t db = db1 + (uint64_t)(((dx * KU + 2 * st) * 3 * N * 16) >> 4);
+            const int now = q == 0 && last == i ? count - 1 : count;  // (without row i's start)
+            const int h = min(now, head);
+            umma_rows_of<N>(h, acc, da, db, true);
+            umma_rows_of<N>(now - h, tmem, da, db + (uint64_t)(h * N), true);
+            if (now < count) umma_rows<N, 1>(tmem + (uint32_t)((i % B) * N), da, db + (uint64_t)(now * N), false);
+          }
+        }
+        if (i >= 2) umma_commit(smem_u32(&ctl.acc_full[(i - 2) % B]));
+        umma_commit(smem_u32(&ctl.empty[i % S]));
+      }
+    }
+  } else {
+    for (int o = 0; o < rows; o++) {
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl.acc_full[o % B]), (uint32_t)((o / B) & 1), fail));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+      const int gx = x0 + warp * 32 + lane;
+      const size_t p = (size_t)(img * a.h + y_begin + o) * a.w + gx;
+      conv_epilogue_row<N>(a, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((o % B) * N), p, gx < a.w, bias_s);
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+      mbar_arrive(smem_u32(&ctl.acc_empty[o % B]));
+    }
+  }
+  conv_ctl_end(ctl, COLS, ok, err);
+}
+
+// Chunked form, for the layers whose weights do not fit: persistent CTAs take
+// tiles of R output rows x 128 pixels; a stage is one chunk of 16 input
+// channels (R + 2 input rows and 9 x 16 x N weights), S stages in the ring, the
+// next tile's first chunks loading under the last ones of this.  B accumulator
+// sets of R rows (2: a tile is stored while the next one's MMAs run).
+template <int N, int R, int S, int B>
+constexpr int conv_tc_smem_bytes() {
+  return S * (2 * (R + 2) * kUnitPitch + 9 * 2 * N * 16) + N * 4 + (int)sizeof(ConvCtl<S, B>) + 16;
+}
+template <int N, int R, int S, int B>
+__global__ void __launch_bounds__(kConvThreads) conv_tc_kernel(const ConvArgs a, int tiles, int* err) {
+  extern __shared__ __align__(128) uint8_t tc_smem[];
+  constexpr int KU = 2, ROWS = R + 2;
+  constexpr int HALO_B = KU * ROWS * kUnitPitch, STAGE_B = HALO_B + 9 * KU * N * 16;
+  constexpr uint32_t LBO_A = ROWS * kUnitPitch;  // next K unit of the staged rows
+  constexpr uint32_t LBO_B = 3 * N * 16;         // next K unit of the weights
+  constexpr int COLS = pow2_cols(B * R * N);
+  constexpr int L = S - 1;                      // chunks in flight
+  const uint32_t ring_a = smem_u32(tc_smem);
+  ConvCtl<S, B>& ctl = *reinterpret_cast<ConvCtl<S, B>*>(tc_smem + S * STAGE_B);
+  float* bias_s = reinterpret_cast<float*>(tc_smem + S * STAGE_B + (sizeof(ConvCtl<S, B>) + 15) / 16 * 16);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tiles_x = (a.w + 127) >> 7, rows_y = (a.h + R - 1) / R;
+  const int chunks = a.cin / 16;
+  for (int i = tid; i < N; i += kConvThreads) bias_s[i] = a.bias && i < a.cout ? a.bias[i] : 0.0f;
+  conv_ctl_init(ctl, COLS);
+  const volatile int* fail = &ctl.fail;
+  const uint32_t tmem = ctl.tmem;
+  bool ok = true;
+  if (warp >= 4 && warp < kMmaWarp) {
+    const int ptid = tid - 128;
+    int n = 0;  // stages begun
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const int x0 = tile % tiles_x * 128, y0 = tile / tiles_x % rows_y * R, img = tile / (tiles_x * rows_y);
+      for (int c = 0; c < chunks; c++, n++) {
+        if (n >= S) ok = mbar_wait(smem_u32(&ctl.empty[n % S]), (uint32_t)((n / S - 1) & 1), fail);
+        if (!ok) break;
+        const uint32_t stage = ring_a + (n % S) * STAGE_B;
+        conv_stage_weights<N, KU>(a, c * 16, stage + HALO_B, ptid);
+        for (int r = 0; r < ROWS; r++) conv_stage_row<KU>(a, img, y0 + r - 1, x0, c * 16, stage + r * kUnitPitch, LBO_A, ptid);
+        cp_commit();
+        if (n >= L) {
+          cp_wait<L>();
+          fence_async();
+          mbar_arrive(smem_u32(&ctl.full[(n - L) % S]));
         }
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar + ((y - y_begin) & 1)))
-                   : "memory");
     }
-    if (y > y_begin) epilogue(y - 1);
+    if (ok) {
+      cp_wait<0>();
+      fence_async();
+      for (int i = max(0, n - L); i < n; i++) mbar_arrive(smem_u32(&ctl.full[i % S]));
+    }
+  } else if (warp == kMmaWarp) {
+    if (lane == 0) {
+      int n = 0, k = 0;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, k++) {
+        if (k >= B) ok = mbar_wait(smem_u32(&ctl.acc_empty[k % B]), (uint32_t)((k / B - 1) & 1), fail);
+        const uint32_t acc0 = tmem + (uint32_t)((k % B) * R * N);
+        for (int c = 0; c < chunks && ok; c++, n++) {
+          ok = mbar_wait(smem_u32(&ctl.full[n % S]), (uint32_t)((n / S) & 1), fail);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+          const uint32_t stage = ring_a + (n % S) * STAGE_B;
+          // descriptors advance by address only (16-byte units in the low bits)
+          const uint64_t da0 = umma_desc(stage, LBO_A, 128), db0 = umma_desc(stage + HALO_B, LBO_B, 128);
+#pragma unroll
+          for (int i = 0; i < ROWS; i++) {  // input row i: output rows i - 2 .. i of the tile
+            const int first = i < 2 ? 0 : i - 2, last = i < R ? i : R - 1;
+#pragma unroll
+            for (int dx = 0; dx < 3; dx++) {
+              const uint64_t da = da0 + (uint64_t)((i * kUnitPitch + dx * 16) >> 4);
+              const uint64_t db = db0 + (uint64_t)(dx * KU * 3 * N + (first - (i - 2)) * N);
+              const uint32_t acc = acc0 + (uint32_t)(first * N);
+              if (dx == 0 && last == i && c == 0) {  // row i's accumulator starts here
+                umma_rows_of<N>(last - first, acc, da, db, true);
+                umma_rows<N, 1>(acc0 + (uint32_t)(i * N), da, db + (uint64_t)((last - first) * N), false);
+              } else {
+                umma_rows_of<N>(last - first + 1, acc, da, db, true);
+              }
+            }
+          }
+          umma_commit(smem_u32(&ctl.empty[n % S]));
+        }
+        if (ok) umma_commit(smem_u32(&ctl.acc_full[k % B]));
+      }
+    }
+  } else {
+    int k = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl.acc_full[k % B]), (uint32_t)((k / B) & 1), fail));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+      const int gx = tile % tiles_x * 128 + warp * 32 + lane, y0 = tile / tiles_x % rows_y * R, img = tile / (tiles_x * rows_y);
+#pragma unroll 1
+      for (int r = 0; r < R; r++) {
+        const size_t p = (size_t)(img * a.h + y0 + r) * a.w + gx;
+        conv_epilogue_row<N>(a, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(((k % B) * R + r) * N), p, gx < a.w && y0 + r < a.h, bias_s);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+      mbar_arrive(smem_u32(&ctl.acc_empty[k % B]));
+    }
   }
-  if (ok && y_end > y_begin) epilogue(y_end - 1);
-  if (!ok && tid == 0) atomicExch(err, 1);
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
-  __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(COLS));
+  conv_ctl_end(ctl, COLS, ok, err);
 }
 
 // ------------------------------------------------------- weight gradient --
@@ -564,13 +666,16 @@ struct WgradArgs {
   int cs;
 };
 
+// Stages of 32 pixels are copied three ahead of the products with cp.async
+// (one stage at a time the kernel waited for every load: four 256x256 crops,
+// the 96 -> 32 layer: 307 -> 221 us); the products of a CTA come in pixel order.
 template <int CI>
-__global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a) {
+__global__ void __launch_bounds__(128) wgrad_kernel(const WgradArgs a) {
   constexpr int KP = 32;   // pixels per stage
-  constexpr int NT = CI / 8;
+  constexpr int NT = CI / 8, ST = 4;
   constexpr int DS = 64 + 8, XS = CI + 8;
-  __shared__ __align__(16) bf16 dys[KP * DS];
-  __shared__ __align__(16) bf16 xs[KP * XS];
+  __shared__ __align__(16) bf16 dys[ST][KP * DS];
+  __shared__ __align__(16) bf16 xs[ST][KP * XS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int co0 = blockIdx.y * 64;
   const int chunks = a.cin / CI;
@@ -582,47 +687,68 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs a) {
   float acc[NT][4];
 #pragma unroll
   for (int i = 0; i < NT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (long pb = p_begin; pb < p_end; pb += KP) {
-    // dY rows: KP pixels x 64 channels
-    for (int v = tid; v < KP * 8; v += 128) {
-      const int r = v >> 3, part = v & 7;
-      const long p = pb + r;
-      const int co = co0 + part * 8;
-      uint4 val = zero;
-      if (p < p_end && co < a.cout) val = *reinterpret_cast<const uint4*>(a.dy + p * a.cout + co);
-      *reinterpret_cast<uint4*>(dys + r * DS + part * 8) = val;
+  // This thread's copies of a stage: dY rows tid / 8 and 16 + tid / 8, part
+  // tid % 8; the shifted X row tid / (CI / 8), part tid % (CI / 8), whose image
+  // position advances with the stages.
+  const int dr = tid >> 3, dpart = tid & 7;
+  const bool dlive = co0 + dpart * 8 < a.cout;
+  const int xr = tid / (CI / 8), xpart = tid - xr * (CI / 8);
+  const bool xmine = xr < KP;
+  long xp = p_begin + xr;
+  int img = (int)(xp / ((long)a.h * a.w)), rem = (int)(xp - (long)img * a.h * a.w);
+  int y = rem / a.w, x = rem - y * a.w;
+  const int stages = (int)((p_end - p_begin + KP - 1) / KP);
+  auto load = [&](int k) {
+    const long pb = p_begin + (long)k * KP;
+    const int s = k % ST;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int r = dr + 16 * h;
+      const bool in = pb + r < p_end && dlive;
+      cp_async16(smem_u32(&dys[s][r * DS + dpart * 8]), in ? a.dy + (pb + r) * a.cout + co0 + dpart * 8 : a.dy, in);
     }
-    // shifted X rows: KP pixels x CI channels
-    for (int v = tid; v < KP * (CI / 8); v += 128) {
-      const int r = v / (CI / 8), part = v - r * (CI / 8);
-      const long p = pb + r;
-      uint4 val = zero;
-      if (p < p_end) {
-        const int img = (int)(p / ((long)a.h * a.w));
-        const int rem = (int)(p - (long)img * a.h * a.w);
-        const int y = rem / a.w + dy, xx = rem % a.w + dx;
-        if (y >= 0 && y < a.h && xx >= 0 && xx < a.w)
-          val = *reinterpret_cast<const uint4*>(conv_in(a.x, a.x2, a.cin, a.cs, a.h, a.w, img, y, xx, ci0 + part * 8));
+    if (xmine) {
+      const int yy = y + dy, xx = x + dx;
+      const bool in = xp < p_end && yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
+      cp_async16(smem_u32(&xs[s][xr * XS + xpart * 8]), in ? conv_in(a.x, a.x2, a.cin, a.cs, a.h, a.w, img, yy, xx, ci0 + xpart * 8) : a.x, in);
+      xp += KP;
+      x += KP;
+      while (x >= a.w) {
+        x -= a.w;
+        if (++y == a.h) {
+          y = 0;
+          img++;
+        }
       }
-      *reinterpret_cast<uint4*>(xs + r * XS + part * 8) = val;
     }
-    __syncthreads();
+  };
+#pragma unroll
+  for (int k = 0; k < ST - 1; k++) {
+    if (k < stages) load(k);
+    cp_commit();
+  }
+  for (int k = 0; k < stages; k++) {
+    cp_wait<ST - 2>();
+    __syncthreads();  // stage k is in, and every warp is done with stage k - 1
+    if (k + ST - 1 < stages) load(k + ST - 1);
+    cp_commit();
+    if (co0 + warp * 16 >= a.cout) continue;  // no output channels for this warp
+    const bf16* ds = dys[k % ST];
+    const bf16* xk = xs[k % ST];
 #pragma unroll
     for (int kb = 0; kb < KP; kb += 16) {
       const int mi = lane >> 3, row = lane & 7;
       uint32_t a0, a1, a2, a3;
       // A[m = co][k = pixel] from dY rows (pixel-major): transposed loads
-      ldsm_x4_t(smem_u32(dys + (kb + (mi >> 1) * 8 + row) * DS + warp * 16 + (mi & 1) * 8), a0, a1, a2, a3);
+      ldsm_x4_t(smem_u32(ds + (kb + (mi >> 1) * 8 + row) * DS + warp * 16 + (mi & 1) * 8), a0, a1, a2, a3);
 #pragma unroll
       for (int nt = 0; nt < NT; nt += 2) {
         uint32_t b0, b1, b2, b3;
-        ldsm_x4_t(smem_u32(xs + (kb + (mi & 1) * 8 + row) * XS + (nt + (mi >> 1)) * 8), b0, b1, b2, b3);
+        ldsm_x4_t(smem_u32(xk + (kb + (mi & 1) * 8 + row) * XS + (nt + (mi >> 1)) * 8), b0, b1, b2, b3);
         mma_bf16(acc[nt], a0, a1, a2, a3, b0, b1);
         mma_bf16(acc[nt + 1], a0, a1, a2, a3, b2, b3);
       }
     }
-    __syncthreads();
   }
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
@@ -660,13 +786,28 @@ __global__ void bgrad_kernel(const bf16* __restrict__ dy, float* __restrict__ db
 }
 
 // g[i] += sum over s = 0 .. splits - 1, in that order, of part[s * n + i]:
-// the partial sums of wgrad_kernel / bgrad_kernel folded in a fixed order.
+// the partial sums of wgrad_kernel folded in a fixed order.
 __global__ void reduce_kernel(const float* __restrict__ part, float* __restrict__ g, long n, int splits) {
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     float s = 0.0f;
     for (int k = 0; k < splits; k++) s += part[(size_t)k * n + i];
     g[i] += s;
   }
+}
+// The same for bgrad_kernel's few channels and many partials, one block per
+// channel: the partials are fetched together and added in order from shared
+// memory (one thread fetching each in turn waited 105 us for 1,184 of them;
+// now 9 us).
+constexpr int kBgradBlocks = 1184;
+__global__ void __launch_bounds__(256) reduce_bias_kernel(const float* __restrict__ part, float* __restrict__ g, int cout, int splits) {
+  __shared__ float v[kBgradBlocks];
+  for (int k = threadIdx.x; k < splits; k += blockDim.x) v[k] = part[(size_t)k * cout + blockIdx.x];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  float s = 0.0f;
+#pragma unroll 16
+  for (int k = 0; k < splits; k++) s += v[k];
+  g[blockIdx.x] += s;
 }
 
 // --------------------------------------------------- pooling and concat --
@@ -1009,79 +1150,79 @@ int launch_conv(const ConvArgs& a, cudaStream_t s) {
   return check_launch("conv_kernel");
 }
 
-// The forward convolutions on tcgen05 (cout 16..128).  R rows per CTA keep
-// R x N TMEM columns within 256, so two CTAs per SM fit the 512 columns.
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  return sms;
+}
 // Shared memory per CTA is padded so that the CTAs one SM can hold never ask
 // for more than its 512 TMEM columns together (an allocation then never
 // waits on another CTA).
-template <int N, int CC, int R>
-constexpr int conv_tc_launch_smem() {
-  constexpr int need = conv_tc_smem_bytes<N, CC, R>();
-  constexpr int floor_b = 228 * 1024 / (512 / pow2_cols(R * N) + 1) + 1024;
+constexpr int conv_smem_padded(int need, int cols) {
+  const int floor_b = 228 * 1024 / (512 / cols + 1) + 1024;
   return need > floor_b ? need : floor_b;
 }
-template <int N, int CC, int R>
-int launch_tc(const ConvArgs& a, int* err, cudaStream_t s) {
-  static_assert(pow2_cols(R * N) <= 256, "TMEM budget");
-  constexpr int smem = conv_tc_launch_smem<N, CC, R>();
-  static_assert(smem <= 227 * 1024, "shared memory per CTA");
-  static bool ready = false;
-  if (!ready) {
-    if (cudaFuncSetAttribute(conv_tc_kernel<N, CC, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return cuda_fail("cudaFuncSetAttribute (conv_tc)", cudaGetLastError());
-    ready = true;
-  }
-  const dim3 grid((unsigned)(((a.w + 127) / 128) * ((a.h + R - 1) / R) * a.n));
-  conv_tc_kernel<N, CC, R><<<grid, 128, smem, s>>>(a, err);
-  count_launch();
-  return check_launch("conv_tc_kernel");
-}
 // Row-streaming launch: rows per CTA chosen so the grid fills the SMs once
-// at the occupancy the shared memory allows (TMEM: 2 x N columns per CTA).
-template <int N, int CIN>
+// at the occupancy the shared memory allows.
+template <int N, int CIN, int S, int B>
 int launch_row(const ConvArgs& a, int* err, cudaStream_t s) {
-  constexpr int need = conv_row_smem_bytes<N, CIN>();
-  constexpr int floor_b = 228 * 1024 / (512 / pow2_cols(2 * N) + 1) + 1024;
-  constexpr int smem = need > floor_b ? need : floor_b;
+  constexpr int smem = conv_smem_padded(conv_row_smem_bytes<N, CIN, S, B>(), pow2_cols(B * N));
   static_assert(smem <= 227 * 1024, "shared memory per CTA");
   static bool ready = false;
   static int sms = 0;
   if (!ready) {
-    if (cudaFuncSetAttribute(conv_row_kernel<N, CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(conv_row_kernel<N, CIN, S, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return cuda_fail("cudaFuncSetAttribute (conv_row)", cudaGetLastError());
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+    sms = device_sms();
     ready = true;
   }
   const int per_sm = std::max(1, 228 * 1024 / (smem + 1024));
+  // One wave: as many row groups per segment as the CTA slots hold (rounded up
+  // instead, 150 groups on 148 SMs took two waves and twice the time).
   const long segs = (long)((a.w + 127) / 128) * a.n;
-  long rows = ((long)a.h * segs + (long)sms * per_sm - 1) / ((long)sms * per_sm);
-  if (rows < 4) rows = 4;
-  if (rows > a.h) rows = a.h;
+  const long want = std::max(1L, (long)sms * per_sm / segs);
+  const long rows = std::min<long>(a.h, std::max(4L, (a.h + want - 1) / want));
   const dim3 grid((unsigned)(segs * ((a.h + rows - 1) / rows)));
-  conv_row_kernel<N, CIN><<<grid, 128, smem, s>>>(a, (int)rows, err);
+  conv_row_kernel<N, CIN, S, B><<<grid, kConvThreads, smem, s>>>(a, (int)rows, err);
   count_launch();
   return check_launch("conv_row_kernel");
+}
+template <int N, int R, int S, int B>
+int launch_tc(const ConvArgs& a, int* err, cudaStream_t s) {
+  constexpr int smem = conv_smem_padded(conv_tc_smem_bytes<N, R, S, B>(), pow2_cols(B * R * N));
+  static_assert(B * R * N <= 512, "TMEM columns");
+  static_assert(smem <= 227 * 1024, "shared memory per CTA");
+  static bool ready = false;
+  static int sms = 0;
+  if (!ready) {
+    if (cudaFuncSetAttribute(conv_tc_kernel<N, R, S, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return cuda_fail("cudaFuncSetAttribute (conv_tc)", cudaGetLastError());
+    sms = device_sms();
+    ready = true;
+  }
+  const int per_sm = std::max(1, 228 * 1024 / (smem + 1024));
+  const int tiles = (a.w + 127) / 128 * ((a.h + R - 1) / R) * a.n;
+  conv_tc_kernel<N, R, S, B><<<std::min(tiles, sms * per_sm), kConvThreads, smem, s>>>(a, tiles, err);
+  count_launch();
+  return check_launch("conv_tc_kernel");
 }
 
 bool tc_shape(const ConvArgs& a) { return a.cout == 16 || a.cout == 32 || a.cout == 64 || a.cout == 96 || a.cout == 128; }
 int launch_conv_tc(const ConvArgs& a, int* err, cudaStream_t s) {
-  // Layers whose weights and a 5-row ring fit in shared memory at 2 or more
-  // CTAs per SM stream rows (measured 11-19 % faster per layer); 96 -> 32,
-  // at 1 CTA per SM, was 2.3x slower that way and keeps the chunked form,
-  // as do the layers whose weights do not fit.
-  if (a.cout == 32 && a.cin == 16) return launch_row<32, 16>(a, err, s);
-  if (a.cout == 32 && a.cin == 32) return launch_row<32, 32>(a, err, s);
-  if (a.cout == 16 && a.cin == 32) return launch_row<16, 32>(a, err, s);
-  if (a.cout == 64 && a.cin == 32) return launch_row<64, 32>(a, err, s);
-  if (a.cout == 64 && a.cin == 64) return launch_row<64, 64>(a, err, s);
-  if (a.cout == 96 && a.cin == 64) return launch_row<96, 64>(a, err, s);
+  // The layers whose weights and a ring of rows fit in shared memory stream
+  // rows; the others take chunks of 16 input channels.
+  if (a.cout == 32 && a.cin == 16) return launch_row<32, 16, 6, 8>(a, err, s);
+  if (a.cout == 32 && a.cin == 32) return launch_row<32, 32, 6, 8>(a, err, s);
+  if (a.cout == 16 && a.cin == 32) return launch_row<16, 32, 6, 8>(a, err, s);
+  if (a.cout == 64 && a.cin == 32) return launch_row<64, 32, 6, 8>(a, err, s);
+  if (a.cout == 64 && a.cin == 64) return launch_row<64, 64, 6, 8>(a, err, s);
+  if (a.cout == 96 && a.cin == 64) return launch_row<96, 64, 5, 5>(a, err, s);
   switch (a.cout) {
-    case 16: return launch_tc<16, 16, 8>(a, err, s);
-    case 32: return launch_tc<32, 16, 8>(a, err, s);
-    case 64: return launch_tc<64, 16, 4>(a, err, s);
-    case 96: return launch_tc<96, 16, 2>(a, err, s);
-    default: return launch_tc<128, 16, 2>(a, err, s);
+    case 16: return launch_tc<16, 8, 4, 2>(a, err, s);
+    case 32: return launch_tc<32, 16, 2, 1>(a, err, s);
+    case 64: return launch_tc<64, 8, 3, 1>(a, err, s);
+    case 96: return launch_tc<96, 4, 4, 1>(a, err, s);
+    default: return launch_tc<128, 2, 4, 2>(a, err, s);
   }
 }
 
@@ -1103,7 +1244,6 @@ long wgrad_max_splits(int cin, int cout) {
   const long base = ((cout + 63) / 64) * 9 * (cin / ci_tile);
   return std::max(1L, 1184 / base) + 1;
 }
-constexpr int kBgradBlocks = 1184;
 
 // dw += the layer's weight gradient: partial sums per pixel range into
 // `part`, then folded in range order (the same sums whatever the schedule).
@@ -1154,7 +1294,9 @@ int cast_weights(arbor_denoiser* d) {
 }
 
 // Forward pass over `features` (batch x h x w x 16 BF16); the output lands in d->out.
-int forward(arbor_denoiser* d, const bf16* features, int batch, int w, int h) {
+// In inference on tcgen05 (base, denoised given) the output layer writes the
+// denoised image itself.
+int forward(arbor_denoiser* d, const bf16* features, int batch, int w, int h, const float4* base = nullptr, float4* denoised = nullptr) {
   cudaStream_t s = d->stream;
   const bf16* in[kActs];
   for (int k = 0; k < kActs; k++) in[k] = d->act[k];
@@ -1164,7 +1306,11 @@ int forward(arbor_denoiser* d, const bf16* features, int batch, int w, int h) {
     const int lv = kAct[kIn[l]].level;
     ConvArgs a{in[kIn[l]], d->wf + d->wf_off[l], d->p + L.boff,
                kOut[l] < 0 ? (void*)d->out : (void*)d->act[kOut[l]], nullptr, L.cin, L.cout, batch, h >> lv, w >> lv, kSpec[l][2],
-               kOut[l] < 0 ? 1 : 0, nullptr, 0};
+               kOut[l] < 0 ? 1 : 0, nullptr, 0, nullptr, nullptr};
+    if (kOut[l] < 0 && d->tc) {
+      a.base = base;
+      a.denoised = denoised;
+    }
     if (kCat[l][0] >= 0) {  // a decoder input: read the skip and the upsampled level below in place
       a.x = d->act[kCat[l][0]];
       a.x2 = d->act[kCat[l][1]];
@@ -1202,7 +1348,7 @@ int backward(arbor_denoiser* d, const bf16* features, int batch, int w, int h) {
     const long px = level_pixels(d, lv, batch, w, h);
     const unsigned blocks = (unsigned)std::min<long>(kBgradBlocks, (px * L.cout + 255) / 256 + 1);
     bgrad_kernel<<<blocks, 256, 0, s>>>(dy, d->part, L.cout, px);
-    reduce_kernel<<<1, 256, 0, s>>>(d->part, d->g + L.boff, L.cout, (int)blocks);
+    reduce_bias_kernel<<<L.cout, 256, 0, s>>>(d->part, d->g + L.boff, L.cout, (int)blocks);
     count_launch(2);
     return check_launch("bgrad_kernel");
   };
@@ -1212,7 +1358,7 @@ int backward(arbor_denoiser* d, const bf16* features, int batch, int w, int h) {
     const LayerParams& L = d->layer[l];
     const int lv = kAct[kIn[l]].level;
     ConvArgs a{dy, d->wb + d->wf_off[l], nullptr, dx, mask_act >= 0 ? d->act[mask_act] : nullptr, L.cout, L.cin, batch, h >> lv, w >> lv, 0, 0,
-               nullptr, 0};
+               nullptr, 0, nullptr, nullptr};
     // tcgen05 where the output width has a tensor-core kernel (all but the
     // 160- and 224-channel decoder inputs); the same K = 16 accumulation order
     // as the mma.sync kernel.
@@ -1535,7 +1681,10 @@ extern "C" int arbor_denoiser_infer(arbor_denoiser* d, const uint16_t* features,
     return ARBOR_ERR_NULL;
   }
   if (int s = check_size("arbor_denoiser_infer", 1, width, height, d)) return s;
-  if (int st = forward(d, reinterpret_cast<const bf16*>(features), 1, width, height)) return st;
+  if (int st = forward(d, reinterpret_cast<const bf16*>(features), 1, width, height, reinterpret_cast<const float4*>(base),
+                       reinterpret_cast<float4*>(denoised)))
+    return st;
+  if (d->tc) return ARBOR_OK;
   const long px = (long)width * height;
   output_kernel<<<ew_grid(px), 256, 0, d->stream>>>(d->out, reinterpret_cast<const float4*>(base), reinterpret_cast<float4*>(denoised), px);
   count_launch();
