@@ -19,13 +19,17 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libarbor_b200.so")
-SOURCES = ["build.cu", "camera.cu", "render.cu", "count.cu", "engine.cu", "batch.cu", "denoise.cu", "scratch.cu"]
+SOURCES = ["build.cu", "camera.cu", "render.cu", "filter.cu", "count.cu", "engine.cu", "batch.cu", "denoise.cu", "scratch.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + [
     "-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-prec-div=true", "-prec-sqrt=true",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "-DARBOR_BUILD", "--expt-relaxed-constexpr",
 ]
+
+# Per-file device-assembler flags: the filter kernels run 1 % faster as ptxas
+# -O1 schedules them (3840x2160 filter+resolve 318 against 321 us).
+FILE_FLAGS = {"filter.cu": ["-Xptxas", "-O1"]}
 
 
 def nvcc() -> str:
@@ -52,7 +56,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         obj = os.path.join(BUILD, src.replace(".cu", ".o"))
         objs.append(obj)
         if force or _stale(obj, [path, __file__] + headers):
-            cmd = [nvcc(), *NVCC_FLAGS, "-c", path, "-o", obj]
+            cmd = [nvcc(), *NVCC_FLAGS, *FILE_FLAGS.get(src, []), "-c", path, "-o", obj]
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             res = subprocess.run(cmd, capture_output=True, text=True)

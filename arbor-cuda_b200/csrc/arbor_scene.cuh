@@ -97,6 +97,8 @@ __device__ __forceinline__ Wood load_wood(const float* P, int id) {
   w.hs731 = hashU((uint32_t)(w.seed + 731));
   return w;
 }
+// noise3 out of line, for the shading's many uses.
+static __device__ __noinline__ float noise3_call(f3 p, int seed) { return noise3(p, seed); }
 // Voronoi bark relief (Arbor.cu:149-169).  fine/grain are the footprint
 // band weights of the 10 mm and 2.5 mm bands (constant per call).
 // kMarch: the SDF march of the intersection test, whose angular terms take
@@ -168,8 +170,8 @@ __device__ __forceinline__ float bark_cut(const Wood& w, f3 p, float fp, float f
   // its noise (8 hashes) is not evaluated.  Primary rays: the 2.5 mm band
   // beyond 2 m, the 10 mm band beyond 8 m at full HD.
   float splinter = 0.5f, pores = 0.5f;
-  if (fine != 0.0f) splinter = noise3(coord, w.seed);
-  if (grain != 0.0f) pores = noise3(coord * 4.0f, w.seed + 731);
+  if (fine != 0.0f) splinter = kMarch ? noise3(coord, w.seed) : noise3_call(coord, w.seed);
+  if (grain != 0.0f) pores = kMarch ? noise3(coord * 4.0f, w.seed + 731) : noise3_call(coord * 4.0f, w.seed + 731);
   return amp * clampf(0.32f + coarse * (plates - 0.37f) * 0.69f + fine * (splinter - 0.5f) * 0.24f + grain * (pores - 0.5f) * 0.08f, 0.005f, 1.0f);
 }
 // Wood SDF (Arbor.cu:170).

@@ -1,6 +1,6 @@
-// render.cu - per-frame image passes: tracePixels, shadePixels,
-// filterLighting, resolvePixels (Arbor.cu:252-304) and their single-tree and
-// fused variants, with their C-ABI entry points.
+// render.cu - per-frame image passes: tracePixels and shadePixels
+// (Arbor.cu:252-289) and their single-tree and species variants, with their
+// C-ABI entry points (filter and resolve: filter.cu).
 //
 // Launch shapes: the trace and the shade's shadow pass are persistent (2
 // CTAs per SM, lanes taking pixels of 8x4 blocks as their rays finish); the
@@ -270,31 +270,6 @@ __global__ void __launch_bounds__(kBlock) shade_inorder_kernel(const float* __re
   reinterpret_cast<float4*>(Guide)[pixel] = make_float4(sh.guide.x, sh.guide.y, sh.guide.z, 1.0f);
 }
 
-// filterLighting (+ resolvePixels) of one 32x16 tile per CTA, its halo
-// staged from global memory; 4 CTAs per SM.
-template <bool kResolve>
-__global__ void __launch_bounds__(kFX * kFT, 4) filter_kernel(const float* __restrict__ Linear, const float* __restrict__ Guide,
-                                                              const float* __restrict__ Hit, float* __restrict__ Filtered,
-                                                              float* __restrict__ History, uint32_t* __restrict__ Pixels,
-                                                              const float* __restrict__ C, int width, int height) {
-  __shared__ FilterTile s;
-  filter_tile<kResolve>(s, Linear, Guide, Hit, Filtered, History, Pixels, kResolve ? C[9] : 0.0f, kResolve ? C[10] : 0.0f, C[15],
-                        kResolve ? C[20] : 0.0f, width, height, blockIdx.x * kFX, blockIdx.y * kFY);
-}
-
-// resolvePixels alone (Arbor.cu:304): 32x8-pixel CTAs, one pixel per thread.
-constexpr int kRX = 32, kRY = 8;
-__global__ void __launch_bounds__(kRX * kRY) resolve_kernel(const float* __restrict__ Filtered, float* __restrict__ History,
-                                                            uint32_t* __restrict__ Pixels, const float* __restrict__ C, int width,
-                                                            int height) {
-  const int x = blockIdx.x * kRX + threadIdx.x, y = blockIdx.y * kRY + threadIdx.y;
-  if (x >= width || y >= height) return;
-  float4 f = __ldg(reinterpret_cast<const float4*>(Filtered) + y * width + x);
-  const float count = sample_count(C[9], C[10]);
-  resolve_px(mk(f.x, f.y, f.z), History, Pixels, count, 1.0f / (count + 1.0f), C[20], vig_coord(x, width), vig_coord(y, height), y * width + x);
-}
-
-
 // Opt a kernel in to kPassSmemTable of dynamic shared memory, once per device.
 inline bool batch_smem_ready(const void* kernel) {
   static const void* done[64][8] = {};
@@ -323,21 +298,6 @@ dim3 pool_grid(int w, int h) {
   const long blocks = (long)((w + 7) / 8) * ((h + 3) / 4);
   return dim3((unsigned)std::min<long>(blocks, 2L * sms[dev]));
 }
-dim3 filter_grid(int w, int h) { return dim3((w + kFX - 1) / kFX, (h + kFY - 1) / kFY); }
-
-// filterLighting (+ resolvePixels) over width x height: one 32x16 tile per CTA.
-int launch_filter(const char* name, bool resolve, const float* Linear, const float* Guide, const float* Hit, float* Filtered, float* History,
-                  uint32_t* Pixels, const float* C, int width, int height, cudaStream_t stream) {
-  if (resolve)
-    filter_kernel<true><<<filter_grid(width, height), dim3(kFX, kFT), 0, stream>>>(Linear, Guide, Hit, Filtered, History, Pixels, C, width, height);
-  else
-    filter_kernel<false><<<filter_grid(width, height), dim3(kFX, kFT), 0, stream>>>(Linear, Guide, Hit, Filtered, nullptr, nullptr, C, width,
-                                                                                    height);
-  count_launch();
-  return check_launch(name);
-}
-dim3 resolve_grid(int w, int h) { return dim3((w + kRX - 1) / kRX, (h + kRY - 1) / kRY); }
-
 // Checks of tracePixels / shadePixels, shared by the entries and the engine.
 int trace_checks(const char* name, const float* P, const float* Nodes, const uint32_t* Order, const float* C, const float* Hit, int width,
                  int height, bool* empty) {
@@ -561,49 +521,3 @@ extern "C" int arbor_shadePixelsInOrder(const float* P, const float* Nodes, cons
   count_launch();
   return check_launch(name);
 }
-extern "C" int arbor_filterLighting(const float* Linear, const float* Guide, const float* Hit, float* Filtered, const float* C, int width,
-                                    int height, arbor_stream stream) {
-  const char* name = "arbor_filterLighting";
-  bool empty;
-  if (int s = check_image(name, width, height, &empty)) return s;
-  size_t img = empty ? 0 : image_bytes(width, height);
-  const Binding b[] = {{Linear, img, false, 16, "Linear"},
-                       {Guide, img, false, 16, "Guide"},
-                       {Hit, img, false, 16, "Hit"},
-                       {Filtered, img, true, 16, "Filtered"},
-                       {C, kC, false, 4, "C"}};
-  if (int s = check_bindings(name, b)) return s;
-  if (empty) return ARBOR_OK;
-  return launch_filter(name, false, Linear, Guide, Hit, Filtered, nullptr, nullptr, C, width, height, stream);
-}
-extern "C" int arbor_resolvePixels(const float* Filtered, float* History, uint32_t* Pixels, const float* C, int width, int height,
-                                   arbor_stream stream) {
-  const char* name = "arbor_resolvePixels";
-  bool empty;
-  if (int s = check_image(name, width, height, &empty)) return s;
-  size_t img = empty ? 0 : image_bytes(width, height);
-  const Binding b[] = {{Filtered, img, false, 16, "Filtered"},
-                       {History, img, true, 16, "History"},
-                       {Pixels, empty ? 0 : pixel_bytes(width, height), true, 4, "Pixels"},
-                       {C, kC, false, 4, "C"}};
-  if (int s = check_bindings(name, b)) return s;
-  if (empty) return ARBOR_OK;
-  resolve_kernel<<<resolve_grid(width, height), dim3(kRX, kRY), 0, stream>>>(Filtered, History, Pixels, C, width, height);
-  count_launch();
-  return check_launch(name);
-}
-extern "C" int arbor_filterResolve(const float* Linear, const float* Guide, const float* Hit, float* Filtered, float* History, uint32_t* Pixels,
-                                   const float* C, int width, int height, arbor_stream stream) {
-  const char* name = "arbor_filterResolve";
-  bool empty;
-  if (int s = check_image(name, width, height, &empty)) return s;
-  size_t img = empty ? 0 : image_bytes(width, height);
-  const Binding b[] = {{Linear, img, false, 16, "Linear"},     {Guide, img, false, 16, "Guide"},
-                       {Hit, img, false, 16, "Hit"},           {Filtered, img, true, 16, "Filtered"},
-                       {History, img, true, 16, "History"},    {Pixels, empty ? 0 : pixel_bytes(width, height), true, 4, "Pixels"},
-                       {C, kC, false, 4, "C"}};
-  if (int s = check_bindings(name, b)) return s;
-  if (empty) return ARBOR_OK;
-  return launch_filter(name, true, Linear, Guide, Hit, Filtered, History, Pixels, C, width, height, stream);
-}
-
