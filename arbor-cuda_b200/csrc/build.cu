@@ -1,15 +1,19 @@
 // build.cu - scene build: growTree, makePrimitives, makeKeys, sortPass,
 // makeBounds, reduceBounds (Arbor.cu:75-142) as drop-in entries, plus the
 // fused build (grow all levels in one CTA; primitives and keys in one pass;
-// a stable LSD radix sort in place of 120 bitonic stages; all 15 BVH levels
+// a stable LSD radix sort (one cluster launch) in place of 120 bitonic stages; all 15 BVH levels
 // in two launches).
 //
 // Generation uses correctly rounded sin/cos/pow (xsin/xcos/xpow) and
 // -fmad=false, so B and P agree with a correctly rounded CPU libm; keys,
 // order and every node depend only on + - * / min max of P and are
 // bit-identical to the reference for identical P.
+#include <cooperative_groups.h>
+
 #include "abi_util.h"
 #include "tight.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace arbor {
 namespace {
@@ -254,79 +258,104 @@ __global__ void __launch_bounds__(128) sort_pass_kernel(uint32_t* __restrict__ K
 }
 
 // ----------------------------------------------------------- radix sort --
-// Stable LSD radix sort of 32768 (key, value) pairs, 8 bits per pass, one
-// launch per pass.  Each of the 16 CTAs ranks 2048 consecutive elements; it
-// obtains the global digit offsets by counting all 32768 digits itself (a
-// 128 KB L2-resident read), so no inter-CTA synchronisation is needed.
-// Ranks within a CTA are stable: warps own consecutive 32-element groups,
-// lanes rank among equal digits with __match_any_sync.
-constexpr int kSortCtas = 16;
+// Stable LSD radix sort of 32768 (key, value) pairs, 8 bits per pass, in one
+// launch: a cluster of 8 CTAs holds the pairs in its shared memory, 4096 per
+// CTA, and passes them on through it.  Per pass each CTA counts its digits, the
+// CTAs read each other's counts, every pair's rank follows, and it is stored
+// into the shared memory of the CTA that holds that rank.  Ranks are stable:
+// warps own consecutive 32-element groups, lanes rank among equal digits with
+// __match_any_sync.  (One launch per pass, in which each CTA counted all 32768
+// digits to need nothing from the others, took 4 x 11 us; this takes 33 us.  The pairs
+// travel as 8-byte stores: as two of 4 bytes it took 41 us.)
+constexpr int kSortCtas = 8;
 constexpr int kSortThreads = 1024;
-constexpr int kSortPerCta = kCapacity / kSortCtas;  // 2048
+constexpr int kSortPerCta = kCapacity / kSortCtas;  // 4096
+struct SortSmem {
+  uint2 pair[2][kSortPerCta];  // key, value
+  uint32_t wcnt[kSortThreads / 32][256];
+  uint32_t hist[256], base[256], scan[8];
+};
 
-__global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                                  uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int shift) {
-  __shared__ uint32_t before[256];
-  __shared__ uint32_t total[256];
-  __shared__ uint32_t base[256];
-  __shared__ uint32_t wcnt[kSortThreads / 32][256];
-  const int tid = threadIdx.x;
-  const int start = blockIdx.x * kSortPerCta;
-  if (tid < 256) {
-    before[tid] = 0;
-    total[tid] = 0;
-  }
-  __syncthreads();
-  for (int e = tid; e < kCapacity; e += kSortThreads) {
-    uint32_t d = (__ldg(kin + e) >> shift) & 255u;
-    atomicAdd(&total[d], 1u);
-    if (e < start) atomicAdd(&before[d], 1u);
-  }
-  __syncthreads();
-  // Exclusive scan of the digit totals (one warp, 8 digits per lane).
-  if (tid < 32) {
-    uint32_t local[8], s = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      local[k] = s;
-      s += total[tid * 8 + k];
-    }
-    uint32_t incl = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
-      if (tid >= o) incl += n;
-    }
-    uint32_t excl = incl - s;
-#pragma unroll
-    for (int k = 0; k < 8; k++) base[tid * 8 + k] = excl + local[k] + before[tid * 8 + k];
-  }
-  const int warp = tid >> 5, lane = tid & 31;
+__global__ void __cluster_dims__(kSortCtas, 1, 1) __launch_bounds__(kSortThreads) radix_sort_kernel(uint32_t* __restrict__ keys,
+                                                                                                    uint32_t* __restrict__ vals) {
+  extern __shared__ __align__(16) uint8_t sort_smem[];
+  SortSmem& s = *reinterpret_cast<SortSmem*>(sort_smem);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank_cta = (int)cluster.block_rank(), start = rank_cta * kSortPerCta;
   const uint32_t lt = (1u << lane) - 1u;
-  for (int round = 0; round < kSortPerCta / kSortThreads; round++) {
-    for (int k = tid; k < (kSortThreads / 32) * 256; k += kSortThreads) (&wcnt[0][0])[k] = 0;
+  for (int e = tid; e < kSortPerCta; e += kSortThreads) {
+    s.pair[0][e] = make_uint2(keys[start + e], vals[start + e]);
+  }
+  __syncthreads();
+  constexpr int kEach = kSortPerCta / kSortThreads;  // a warp owns 32 kEach consecutive pairs
+  for (int pass = 0; pass < 4; pass++) {
+    const int shift = pass * 8, from = pass & 1;
+#pragma unroll
+    for (int k = 0; k < 8; k++) s.wcnt[warp][k * 32 + lane] = 0;
+    __syncwarp();
+    uint2 pair[kEach];
+    uint32_t rank[kEach];
+#pragma unroll
+    for (int r = 0; r < kEach; r++) {
+      const int e = (warp * kEach + r) * 32 + lane;
+      pair[r] = s.pair[from][e];
+      const uint32_t d = (pair[r].x >> shift) & 255u;
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t seen = s.wcnt[warp][d];
+      rank[r] = seen + (uint32_t)__popc(peers & lt);
+      __syncwarp();
+      if ((peers & lt) == 0u) s.wcnt[warp][d] = seen + (uint32_t)__popc(peers);
+      __syncwarp();
+    }
     __syncthreads();
-    int e = start + round * kSortThreads + tid;
-    uint32_t key = __ldg(kin + e), val = __ldg(vin + e);
-    uint32_t d = (key >> shift) & 255u;
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
-    uint32_t rank = __popc(peers & lt);
-    if (rank == 0) wcnt[warp][d] = __popc(peers);
+    if (tid < 256) {  // per digit: each warp's first rank in the CTA, and the CTA's count
+      uint32_t c[kSortThreads / 32], run = 0;
+#pragma unroll
+      for (int w = 0; w < kSortThreads / 32; w++) c[w] = s.wcnt[w][tid];
+#pragma unroll
+      for (int w = 0; w < kSortThreads / 32; w++) {
+        s.wcnt[w][tid] = run;
+        run += c[w];
+      }
+      s.hist[tid] = run;
+    }
+    cluster.sync();  // every CTA's counts are in place
+    uint32_t total = 0, before = 0, incl = 0;
+    if (tid < 256) {
+#pragma unroll
+      for (int r = 0; r < kSortCtas; r++) {
+        const uint32_t c = cluster.map_shared_rank(s.hist, r)[tid];
+        before += r < rank_cta ? c : 0u;
+        total += c;
+      }
+      incl = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+      }
+      if (lane == 31) s.scan[warp] = incl;
+    }
     __syncthreads();
     if (tid < 256) {
-      uint32_t run = base[tid];
-      for (int w = 0; w < kSortThreads / 32; w++) {
-        uint32_t c = wcnt[w][tid];
-        wcnt[w][tid] = run;
-        run += c;
-      }
-      base[tid] = run;
+      uint32_t off = 0;
+      for (int w = 0; w < warp; w++) off += s.scan[w];
+      s.base[tid] = off + incl - total + before;
     }
     __syncthreads();
-    uint32_t pos = wcnt[warp][d] + rank;
-    kout[pos] = key;
-    vout[pos] = val;
-    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kEach; r++) {
+      const uint32_t d = (pair[r].x >> shift) & 255u;
+      const uint32_t pos = s.base[d] + s.wcnt[warp][d] + rank[r], to = pos / kSortPerCta, at = pos % kSortPerCta;
+      cluster.map_shared_rank(s.pair[from ^ 1], to)[at] = pair[r];
+    }
+    cluster.sync();  // the pairs are where the next pass reads them, and the counts have been read
+  }
+  for (int e = tid; e < kSortPerCta; e += kSortThreads) {
+    const uint2 p = s.pair[0][e];
+    keys[start + e] = p.x;
+    vals[start + e] = p.y;
   }
 }
 
@@ -406,14 +435,20 @@ int grid_of(int n, int block) { return (n + block - 1) / block; }
 }  // namespace
 
 // Host helpers reused by the engine and the fused build.
-int launch_sort(uint32_t* Keys, uint32_t* Order, void* scratch, cudaStream_t stream) {
-  uint32_t* k2 = static_cast<uint32_t*>(scratch);
-  uint32_t* v2 = k2 + kCapacity;
-  for (int pass = 0; pass < 4; pass++) {
-    bool even = (pass & 1) == 0;
-    radix_pass_kernel<<<kSortCtas, kSortThreads, 0, stream>>>(even ? Keys : k2, even ? Order : v2, even ? k2 : Keys, even ? v2 : Order, pass * 8);
+int launch_sort(uint32_t* Keys, uint32_t* Order, cudaStream_t stream) {
+  static bool ready[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  if (!ready[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(radix_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+    if (e != cudaSuccess) {
+      set_error("arbor_sortKeys: cannot reserve %zu bytes of shared memory per CTA: %s", sizeof(SortSmem), cudaGetErrorString(e));
+      return ARBOR_ERR_CUDA;
+    }
+    ready[dev] = true;
   }
-  count_launch(4);
+  radix_sort_kernel<<<kSortCtas, kSortThreads, sizeof(SortSmem), stream>>>(Keys, Order);
+  count_launch();
   return check_launch("arbor_sortKeys");
 }
 int launch_bounds_build(const float* P, const uint32_t* Order, float* Nodes, cudaStream_t stream) {
@@ -493,7 +528,7 @@ extern "C" size_t arbor_sort_scratch_bytes(void) { return 2u * kCapacity * sizeo
 extern "C" int arbor_sortKeys(uint32_t* Keys, uint32_t* Order, void* scratch, arbor_stream stream) {
   const Binding b[] = {{Keys, kKeys, true, 4, "Keys"}, {Order, kKeys, true, 4, "Order"}, {scratch, arbor_sort_scratch_bytes(), true, 4, "scratch"}};
   if (int s = check_bindings("arbor_sortKeys", b)) return s;
-  return launch_sort(Keys, Order, scratch, stream);
+  return launch_sort(Keys, Order, stream);
 }
 extern "C" int arbor_buildBounds(const float* P, const uint32_t* Order, float* Nodes, arbor_stream stream) {
   const Binding b[] = {{P, kP, false, 16, "P"}, {Order, kKeys, false, 4, "Order"}, {Nodes, kNodes, true, 16, "Nodes"}};
@@ -518,7 +553,7 @@ extern "C" int arbor_buildScene(int seed, float* B, float* P, uint32_t* Keys, ui
   register_world_seed(seed, stream);  // a forest built from `seed` has world seed `seed` (initCamera sets C[31])
   if (int s = launch_grow_all(B, seed, stream)) return s;
   if (int s = launch_prims_keys(B, P, Keys, Order, seed, stream)) return s;
-  if (int s = launch_sort(Keys, Order, scratch, stream)) return s;
+  if (int s = launch_sort(Keys, Order, stream)) return s;
   if (int s = launch_bounds_build(P, Order, Nodes, stream)) return s;
   if (C != nullptr) return arbor_initCamera(C, P, seed, stream);
   return ARBOR_OK;
@@ -544,22 +579,25 @@ namespace {
 constexpr int kNoAllocMaxPairs = kCapacity;  // largest count the array holds
 static __device__ __align__(256) uint32_t g_noalloc_sort_scratch[2 * kNoAllocMaxPairs];
 
-// One 8-bit LSD pass over the first n pairs (n <= kNoAllocMaxPairs), the
-// same stable ranking as radix_pass_kernel with the tail beyond n masked.
-__global__ void __launch_bounds__(kSortThreads) radix_pass_n_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+constexpr int kPassThreads = 1024, kPassPerCta = 2048;
+// One 8-bit LSD pass over the first n pairs (n <= kNoAllocMaxPairs),
+// stable: each CTA ranks 2048 consecutive elements and counts all n digits
+// itself, so no inter-CTA synchronisation is needed; the tail beyond n is
+// masked.
+__global__ void __launch_bounds__(kPassThreads) radix_pass_n_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                                     uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int shift, int n) {
   __shared__ uint32_t before[256];
   __shared__ uint32_t total[256];
   __shared__ uint32_t base[256];
-  __shared__ uint32_t wcnt[kSortThreads / 32][256];
+  __shared__ uint32_t wcnt[kPassThreads / 32][256];
   const int tid = threadIdx.x;
-  const int start = blockIdx.x * kSortPerCta;
+  const int start = blockIdx.x * kPassPerCta;
   if (tid < 256) {
     before[tid] = 0;
     total[tid] = 0;
   }
   __syncthreads();
-  for (int e = tid; e < n; e += kSortThreads) {
+  for (int e = tid; e < n; e += kPassThreads) {
     uint32_t d = (__ldg(kin + e) >> shift) & 255u;
     atomicAdd(&total[d], 1u);
     if (e < start) atomicAdd(&before[d], 1u);
@@ -584,10 +622,10 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_n_kernel(const uint32
   }
   const int warp = tid >> 5, lane = tid & 31;
   const uint32_t lt = (1u << lane) - 1u;
-  for (int round = 0; round < kSortPerCta / kSortThreads; round++) {
-    for (int k = tid; k < (kSortThreads / 32) * 256; k += kSortThreads) (&wcnt[0][0])[k] = 0;
+  for (int round = 0; round < kPassPerCta / kPassThreads; round++) {
+    for (int k = tid; k < (kPassThreads / 32) * 256; k += kPassThreads) (&wcnt[0][0])[k] = 0;
     __syncthreads();
-    int e = start + round * kSortThreads + tid;
+    int e = start + round * kPassThreads + tid;
     bool live = e < n;
     uint32_t key = live ? __ldg(kin + e) : 0u, val = live ? __ldg(vin + e) : 0u;
     uint32_t d = live ? ((key >> shift) & 255u) : 256u;  // 256 marks the masked tail
@@ -597,7 +635,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_n_kernel(const uint32
     __syncthreads();
     if (tid < 256) {
       uint32_t run = base[tid];
-      for (int w = 0; w < kSortThreads / 32; w++) {
+      for (int w = 0; w < kPassThreads / 32; w++) {
         uint32_t c = wcnt[w][tid];
         wcnt[w][tid] = run;
         run += c;
@@ -671,10 +709,10 @@ extern "C" int arbor_sortKeysNoAlloc(uint32_t* Keys, uint32_t* Order, int count,
   if (int s = noalloc_scratch(stream, &scratch)) return s;
   uint32_t* k2 = scratch;
   uint32_t* v2 = scratch + kNoAllocMaxPairs;
-  int ctas = (count + kSortPerCta - 1) / kSortPerCta;
+  int ctas = (count + kPassPerCta - 1) / kPassPerCta;
   for (int pass = 0; pass < 4; pass++) {
     bool even = (pass & 1) == 0;
-    radix_pass_n_kernel<<<ctas, kSortThreads, 0, stream>>>(even ? Keys : k2, even ? Order : v2, even ? k2 : Keys, even ? v2 : Order, pass * 8,
+    radix_pass_n_kernel<<<ctas, kPassThreads, 0, stream>>>(even ? Keys : k2, even ? Order : v2, even ? k2 : Keys, even ? v2 : Order, pass * 8,
                                                            count);
   }
   count_launch(4);

@@ -26,7 +26,6 @@ void set_error(const char* fmt, ...) {
 }
 std::atomic<uint64_t>& launch_counter() { return g_launches; }
 
-int launch_sort(uint32_t* Keys, uint32_t* Order, void* scratch, cudaStream_t stream);
 
 }  // namespace arbor
 
