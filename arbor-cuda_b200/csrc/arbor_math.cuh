@@ -219,7 +219,7 @@ __device__ __forceinline__ Instance make_instance(int tree, int ws) {
 // table built from them; block prologues take the values from it, and the
 // persistent trace and shadow passes read the slot's table in place (global
 // memory, L1/L2-resident) instead of building one in shared memory, which
-// leaves their warp batches the room for deeper queues.  A seed without a
+// leaves their block batches the room.  A seed without a
 // slot keeps make_instance's values.
 constexpr int kTrigSlots = 64;
 struct WorldTrig {

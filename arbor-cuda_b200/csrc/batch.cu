@@ -7,7 +7,7 @@
 //                             instance table and the filter/resolve scalars
 //                             of its C record; resets the queues; per scene:
 //                             the tight boxes the passes traverse (tight.cuh)
-//   batch_pool_kernel<trace>  persistent warps walk the views; in each, their
+//   batch_pool_kernel<trace>  persistent CTAs walk the views; in each, their
 //                             lanes take pixels from the view's own queue as
 //                             their rays finish and run tracePixels
 //                             (Arbor.cu:252)
@@ -24,12 +24,12 @@
 // single-image entries (passes.cuh), so a view renders as
 // arbor_tracePixels + arbor_shadePixels + arbor_filterResolve render it with
 // the same C, apart from the order in which exactly equal hit distances are
-// met (the warp batch groups rays by tile; see warpbatch.cuh).
+// met (see blockbatch.cuh).
 //
 // The autotuner times the trace, shadow and compose kernels on a sample of
 // the views for each compose tile shape (16x16 or 32x8), CTAs per SM (1 or
-// 2), view order (as given, or the largest views first) and warp-batch queue
-// depth (12 or 16 candidates per lane), and keeps the fastest.
+// 2), view order (as given, or the largest views first) and chunk of
+// order-dependent trees (12 or 16 candidates), and keeps the fastest.
 #include <algorithm>
 #include <cstring>
 #include <new>
@@ -97,10 +97,9 @@ __global__ void __launch_bounds__(kBlock) batch_setup_kernel(const float* __rest
 }
 
 // tracePixels (kShadow false) or the shadow segments of shadePixels (true,
-// visibility into Linear) of every listed view.  Each warp walks the views in
+// visibility into Linear) of every listed view.  Each CTA walks the views in
 // order and joins each one's pixel queue; its lanes take the view's next
-// pixels as their rays finish, so warps of any CTA share a view's work and
-// move on independently.  The view's camera and instance table are read from
+// pixels as their rays finish, so all CTAs share a view's work.  The view's camera and instance table are read from
 // global memory (the values setup wrote).
 template <int Q, bool kShadow>
 __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* __restrict__ views, const Camera* __restrict__ cams,

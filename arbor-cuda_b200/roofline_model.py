@@ -77,7 +77,7 @@ def flops(counts: dict) -> int:
 # dram__bytes_write.sum) on one 960x544 launch of the forest walk's first
 # frame (seed 7, cold caches): the trace kernel moved 5.33 MB for 522,240
 # primary rays, the shadow pass of shadePixels 20.31 MB for 522,240 pixels
-# (warp-batch queue depth 12).
+# (before the tight boxes; those add 0.8 MB per launch).
 # The 5.7 MB scene stays in L2, so the traffic grows with the pixel count;
 # bench lines scale these to their launch.
 TRACE_DRAM_BYTES_PER_RAY = 10.2

@@ -398,7 +398,7 @@ def measure_workload(args, spec: dict, rank: int, world: int, local_rank: int) -
                          "frac": round(fr_gbs / hbm_peak, 4) if hbm_peak else None, "traffic": None,
                          "algorithmic_bytes": fr_bytes, "peak_source": hbm_source},
         "roofline_build": None if not ms_build else {
-            "kernel": "buildScene (growth, primitives + keys, 4 radix passes, bounds)", "bound": "hbm",
+            "kernel": "buildScene (growth, primitives + keys, radix sort, bounds)", "bound": "hbm",
             "achieved": round(BUILD_BYTES / (ms_build / 1e3) / 1e9, 1), "peak": hbm_peak, "unit": "GB/s",
             "frac": round(BUILD_BYTES / (ms_build / 1e3) / 1e9 / hbm_peak, 4) if hbm_peak else None, "traffic": None,
             "algorithmic_bytes": BUILD_BYTES, "ms_per_build": round(ms_build, 4),
