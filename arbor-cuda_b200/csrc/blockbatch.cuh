@@ -54,6 +54,7 @@ struct BlockBatchOf {
   float4 rayI[kThreads];           // inverse direction and, during the tests, Ray::lbest
   float nearest[kThreads];         // nearest t so far, the entry of its box, and the second nearest candidate's t
   float entry[kThreads], second[kThreads];
+  float slack[kThreads];           // primary rays: by how much a hit may precede its box (enter_tree)
   uint32_t sib[kLeafDepth + 1][3][kThreads];  // deferred nodes (tree_pop)
   LeafSolve solve[kSolves];
   float span[kJobs];               // a candidate's box entry distance (queue place k of thread t: k * kThreads + t)
@@ -154,7 +155,7 @@ __device__ __forceinline__ void block_tests(const TraceCtx& c, BB& b, int n_leaf
         const float4 o = b.rayO[owner], d = b.rayD[owner];
         int steps = c.refine ? b.steps[q] : 0;
         b.res[q] = other_t(scene_P(c, c.species ? b.rayS[owner] : 0), b.prim[q], xyz(o), xyz(d), candidate_footprint(b, q), c.refine,
-                           b.rayI[owner].w, -b.res[q], steps, kMarchRun);
+                           b.rayI[owner].w, -b.res[q], steps, n_other + n_leaf <= 64 ? 64 : kMarchRun);
         if (c.refine) b.steps[q] = (uint8_t)steps;
       }
     } else {
@@ -228,7 +229,7 @@ __device__ __forceinline__ void block_apply(const TraceCtx& c, Ray& r, BB& b, in
   b.nearest[tid] = best;
   b.second[tid] = second;
   b.entry[tid] = entry;
-  r.lbest = fmaxf(best, entry);
+  r.lbest = fmaxf(best, entry) + (c.refine ? b.slack[tid] : 0.0f);
 }
 
 // The pixels of a persistent CTA: the 8x4-pixel blocks blockIdx.x,

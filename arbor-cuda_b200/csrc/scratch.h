@@ -14,7 +14,7 @@ namespace arbor {
 // keeps at most kScratchKeep bytes when nothing uses it; calls on several
 // threads and streams each have their own block.
 constexpr int kTightMaxScenes = 32;
-constexpr size_t kScratchKeep = size_t(32) << 20;
+constexpr size_t kScratchKeep = size_t(56) << 20;
 struct TightScratch {
   uint32_t* boxes = nullptr;
   int status = 0;

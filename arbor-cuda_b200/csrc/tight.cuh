@@ -9,7 +9,7 @@
 // same heap: leaf records bounded by their oriented blade box, inner nodes by
 // the union of their children, everything else as in Nodes.  The boxes are
 // made from P, Order and Nodes by one small kernel in front of each pass (64
-// CTAs per scene, about 6 MB of traffic) and kept nowhere.
+// CTAs per scene, about 7 MB of traffic) and kept nowhere.
 //
 // Why no result changes.  A primitive counts only when the ray passes its box
 // in Nodes, and that test is still made, exactly, on every candidate
@@ -25,6 +25,14 @@
 //    radians (load_leaf), which moves a point of it by at most that times its
 //    distance from the stem base (`reach`).
 // Pruning is by the widened box's entry, which no reported t can precede.
+//
+// The margin grows with the distance and the boxes' own size does not: from
+// about 80 m on a widened tight box is larger than the box in Nodes, whose test
+// needs no margin.  So the boxes of Nodes are stored too, the same way, and a
+// primary ray takes, tree by tree, the tight ones up to a margin of kTightMost
+// and those of Nodes beyond (1080p trace 6.4 -> 5.4 ms, 5.7 with the line at
+// 0.05 m and 5.6 at 0.20; small frames that look along the canopy were up to 1.7
+// times slower with tight boxes at every distance).
 //
 // The boxes are stored 16 bits a coordinate, on a grid over the root's box and
 // rounded outward: the four nodes 4g .. 4g + 3 that a traversal step tests
@@ -45,12 +53,14 @@ namespace arbor {
 
 constexpr int kTightParts = 64;                          // CTAs per scene; part k owns the subtree of node 64 + k
 constexpr int kTightLeaves = kCapacity / kTightParts;    // 512 leaves each; nodes above the parts keep their box
-constexpr int kTightReach = kNodeCount * 3;              // per part its reach (-1: use Nodes), after the nodes' 3 words each
+constexpr int kNodeBoxes = kNodeCount * 3;               // the boxes of Nodes on the same grid, after the tight ones' 3 words each
+constexpr int kTightReach = 2 * kNodeBoxes;              // then per part its reach (-1: use Nodes)
 constexpr int kTightGrid = kTightReach + kTightParts;    // the grid's origin and step (x, y, z each)
 constexpr int kTightWords = kTightGrid + 8;              // words per scene
 constexpr size_t kTightBytes = sizeof(uint32_t) * kTightWords;
 static_assert(kTightWords % 4 == 0, "16-byte aligned groups in every scene");
 constexpr float kTightRel = 1.3e-3f;
+constexpr float kTightMost = 0.10f;  // the widest margin at which the tight boxes are the smaller ones
 constexpr float kSwing = 0.156f;  // wind's largest turn per unit (0.11 + 0.045 radians, rounded up)
 
 struct TightPart {
@@ -159,6 +169,7 @@ __device__ __forceinline__ void tight_build_part(TightPart& s, const float* __re
     s.lo[k] = lo;
     s.hi[k] = hi;
     store_tight(T, node, g, lo, hi);
+    store_tight(T + kNodeBoxes, node, g, nlo, nhi);
   }
   // Nodes' inner nodes: the unions of their children?  (part 0 also looks at
   // the nodes above the parts)
@@ -168,12 +179,16 @@ __device__ __forceinline__ void tight_build_part(TightPart& s, const float* __re
       const int node = ((kTightParts + part) << depth) + (k - (1 << depth));
       float4 plo, phi;
       merge(ldg4(Nodes, 4 * node), ldg4(Nodes, 4 * node + 1), ldg4(Nodes, 4 * node + 2), ldg4(Nodes, 4 * node + 3), plo, phi);
-      bad |= !same_box(plo, phi, ldg4(Nodes, 2 * node), ldg4(Nodes, 2 * node + 1));
+      const float4 nlo = ldg4(Nodes, 2 * node), nhi = ldg4(Nodes, 2 * node + 1);
+      bad |= !same_box(plo, phi, nlo, nhi);
+      store_tight(T + kNodeBoxes, node, g, nlo, nhi);
     }
   }
   if (part == 0 && tid < kTightParts) {
     const float4 lo = ldg4(Nodes, 2 * tid), hi = ldg4(Nodes, 2 * tid + 1);
-    store_tight(T, tid, g, tid > 1 ? lo : make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi);  // 0 and 1 are no one's children: empty
+    const float4 l = tid > 1 ? lo : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // 0 and 1 are no one's children: empty
+    store_tight(T, tid, g, l, hi);
+    store_tight(T + kNodeBoxes, tid, g, l, hi);
     if (tid > 0) {
       float4 plo, phi;
       merge(ldg4(Nodes, 4 * tid), ldg4(Nodes, 4 * tid + 1), ldg4(Nodes, 4 * tid + 2), ldg4(Nodes, 4 * tid + 3), plo, phi);

@@ -56,7 +56,8 @@ struct Ray {
   int tree;
   f3 inv, on, of;   // a box plane at grid coordinate q is met at q * inv - on (near side) or - of (far side)
   uint32_t near;    // per axis a bit: the near plane is the box's hi plane
-  float lbest, lsc; // lbest: the nearest t so far, or its box entry where that lies beyond it (prunes the traversal)
+  int boxes;        // the stored boxes in use: 0 the tight ones, kNodeBoxes those of Nodes
+  float lbest, lsc; // lbest prunes the traversal: the nearest t so far, or its box entry where that lies beyond it, plus the slack
   int lfound;       // its leaf slot, -1, or kMissCounts
   int group, depth; // nodes 4 group .. 4 group + 3 are tested next; depth 0-7 (nodes at heap level 2 depth + 1)
   uint32_t pending; // deferred nodes per depth, 4 bits each
@@ -127,7 +128,21 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
   // again exactly).
   const f3 far = max3(mk(fabsf(lo.x - lro.x), fabsf(lo.y - lro.y), fabsf(lo.z - lro.z)), mk(fabsf(hi.x - lro.x), fabsf(hi.y - lro.y), fabsf(hi.z - lro.z)));
   const float d = length3(far);
-  float m = c.tight.rel * d + c.tight.abs + 1.0e-6f * (d + fabsf(lro.x) + fabsf(lro.y) + fabsf(lro.z));
+  float m = c.tight.rel * d + c.tight.abs;
+  float slack = 0.0f;
+  r.boxes = 0;
+  if (c.refine && m > kTightMost) {  // (a shadow segment's 36 m stay below it)
+    // The boxes are not widened, but a hit may still come before its box by
+    // the margin: pruning allows for it.
+    slack = m;
+    m = 0.0f;
+    r.boxes = kNodeBoxes;
+  }
+  if (c.refine) {
+    b.slack[lane] = slack;
+    r.lbest += slack;
+  }
+  m += 1.0e-6f * (d + fabsf(lro.x) + fabsf(lro.y) + fabsf(lro.z));
   f3 origin = mk(0.0f, 0.0f, 0.0f), step = mk(1.0f, 1.0f, 1.0f);
   if (c.tight.T != nullptr) {
     const float* grid = reinterpret_cast<const float*>(scene_tight(c, r.species)) + kTightGrid;
@@ -308,6 +323,7 @@ template <class WB>
 __device__ __forceinline__ void finish_tree(const TraceCtx& c, Ray& r, WB& b, int lane) {
   if (r.lfound == kMissCounts) {
     r.lfound = first_leaf(scene_nodes(c, r.species), xyz(b.rayO[lane]), xyz(b.rayI[lane]));
+    r.lbest = kFar;
   } else if (r.lfound >= 0) {
     r.lbest = b.nearest[lane];
     // The hit comes before its own box, and another one before that box too:
@@ -487,7 +503,7 @@ __device__ __forceinline__ void tree_step(const TraceCtx& c, Ray& r, WB& b, int 
   float tn[4];       // entries
   uint32_t key[4];   // sort keys, 0xffffffff: rejected
   if (c.tight.T != nullptr) {
-    const uint4* boxes = reinterpret_cast<const uint4*>(scene_tight(c, r.species)) + 3 * r.group;
+    const uint4* boxes = reinterpret_cast<const uint4*>(scene_tight(c, r.species) + r.boxes) + 3 * r.group;
     const uint4 w0 = __ldg(boxes), w1 = __ldg(boxes + 1), w2 = __ldg(boxes + 2);
     const uint32_t w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
     const uint32_t nx = r.near & 1u ? kHalfHi : kHalfLo, ny = r.near & 2u ? kHalfHi : kHalfLo, nz = r.near & 4u ? kHalfHi : kHalfLo;
