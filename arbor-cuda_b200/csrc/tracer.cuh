@@ -324,11 +324,11 @@ __device__ __forceinline__ void finish_tree(const TraceCtx& c, Ray& r, WB& b, in
   if (r.lfound == kMissCounts) {
     r.lfound = first_leaf(scene_nodes(c, r.species), xyz(b.rayO[lane]), xyz(b.rayI[lane]));
     r.lbest = kFar;
-  } else if (r.lfound >= 0) {
-    r.lbest = b.nearest[lane];
+  } else {
+    r.lbest = b.nearest[lane];  // (in place of the traversal's, which holds the slack)
     // The hit comes before its own box, and another one before that box too:
     // which of them a traversal keeps depends on its order.
-    if (b.entry[lane] > r.lbest && b.second[lane] <= b.entry[lane]) {
+    if (r.lfound >= 0 && b.entry[lane] > r.lbest && b.second[lane] <= b.entry[lane]) {
       const TreeResult h = tree_in_order(scene_P(c, r.species), scene_nodes(c, r.species), scene_order(c, r.species), b.rayO[lane], b.rayD[lane],
                                          xyz(b.rayI[lane]), c.wind, r.best / r.lsc, c.refine, WB::kOrdered);
       r.lbest = h.t;

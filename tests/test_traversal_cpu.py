@@ -1,0 +1,126 @@
+"""The batched traversal's device code on the CPU (tests/emu) against the
+reference's traversal as written, on scenes that no seed grows: a few records
+that are small beside the viewing distance, leaves wider than they are long,
+boxes that are inside out.
+
+Bars: no load outside a scene's buffers, and the same hit (t, record and tree)
+bit for bit.  The scenes have no two surfaces close enough along a ray for the
+order of the tests to matter (one that rounding puts before its own box with
+another between the two), so nothing else may differ.
+"""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "arbor-cuda_b200", "csrc")
+CAPACITY, NODE_COUNT, FAR = 32768, 65536, 100000.0
+
+
+def _p(a):
+    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
+
+
+@pytest.fixture(scope="module")
+def emu(tmp_path_factory):
+    gxx, nvcc = shutil.which("g++"), shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    out = str(tmp_path_factory.mktemp("emu") / "traversal.so")
+    subprocess.run([gxx, "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-I", include, "-I", CSRC,
+                    os.path.join(HERE, "emu", "traversal.cpp"), "-o", out], check=True)
+    lib = ctypes.CDLL(out)
+    lib.emu_boxes.restype = lib.emu_trace.restype = ctypes.c_long
+    return lib
+
+
+class Scene:
+    """Records in places 0 .. n - 1 of P (the rest unused), Nodes as
+    arbor_buildBounds makes them."""
+
+    def __init__(self, emu, records):
+        self.emu = emu
+        P = np.zeros((CAPACITY, 24), np.float32)
+        P[:, 3] = -1.0
+        for k, rec in enumerate(records):
+            P[k] = rec
+        self.P, self.Order = P.reshape(-1), np.arange(CAPACITY, dtype=np.uint32)
+        self.Nodes = np.zeros(NODE_COUNT * 8, np.float32)
+        emu.emu_leaf_nodes(_p(self.P), _p(self.Order), _p(self.Nodes))
+        self.T = np.zeros(emu.emu_words(), np.uint32)
+        assert emu.emu_boxes(_p(self.P), _p(self.Order), _p(self.Nodes), _p(self.T)) == 0
+
+    def both(self, rays, wind=0.0, refine=True, inst=None, cone=1.0e-3, time=3.25):
+        """(t, id, tree) of every ray from the block batch and from the
+        reference's traversal; checks that no load left the buffers."""
+        rays = np.ascontiguousarray(rays, np.float32)
+        n, f = len(rays), ctypes.c_float
+        got, want = np.full((n, 3), np.nan, np.float32), np.full((n, 3), np.nan, np.float32)
+        regular = ctypes.c_int(-1)
+        bad = self.emu.emu_trace(_p(self.P), _p(self.Order), _p(self.Nodes), _p(self.T), _p(inst), _p(rays), n, f(cone), f(time), f(wind),
+                                 int(refine), _p(got), ctypes.byref(regular))
+        self.emu.emu_reference(_p(self.P), _p(self.Order), _p(self.Nodes), _p(inst), _p(rays), n, f(cone), f(time), f(wind), int(refine),
+                               _p(want))
+        assert bad == 0, f"{bad} loads outside the scene's buffers"
+        return got, want, regular.value
+
+
+def same(got, want):
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), f"{(got != want).any(1).sum()} of {len(got)} rays differ"
+
+
+def stone(x, y, z, a, b=None, c=None):
+    r = np.zeros(24, np.float32)
+    r[0:4], r[4:7] = (x, y, z, 2.0), (a, b or a, c or a)
+    r[15] = 5.0
+    return r
+
+
+def wood(a, b, ra, rb):
+    r = np.zeros(24, np.float32)
+    r[0:3], r[3], r[4:7], r[7] = a, 0.0, b, ra
+    r[8:11], r[11], r[15], r[18] = (0.0, 0.0, 1.0), rb, 11.0, ra
+    return r
+
+
+def leaf(x, y, z, length, width, stem=0.03, curl=0.02, twist=0.03, frame=((1, 0, 0), (0, 0, 1), (0, 1, 0))):
+    r = np.zeros(24, np.float32)
+    r[0:4], r[4:7], r[7] = (x, y, z, 1.0), frame[0], length
+    r[8:11], r[11], r[12:15], r[15] = frame[1], width, frame[2], 9.0
+    r[16:19] = stem, curl, twist
+    return r
+
+
+def rays_at(target, spread, distance, n, seed, best=FAR):
+    """n rays from points `distance` away toward points within `spread` of the
+    target."""
+    r = np.random.RandomState(seed)
+    d = r.standard_normal((n, 3))
+    d[:, 1] = np.abs(d[:, 1]) + 0.3
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = np.asarray(target) + distance * d
+    at = np.asarray(target) + spread * (2.0 * r.random((n, 3)) - 1.0)
+    v = at - o
+    v /= np.linalg.norm(v, axis=1, keepdims=True)
+    return np.concatenate([o, v, np.full((n, 1), best)], 1)
+
+
+# The scene of the far cases: 2 m high, a few surfaces far apart.
+FAR_SCENE = [wood((0.0, 0.0, 0.0), (0.0, 2.0, 0.0), 0.1, 0.05), leaf(0.3, 1.5, 0.2, 0.2, 0.08), stone(-0.6, 0.2, 0.5, 0.3)]
+
+
+@pytest.mark.parametrize("wind", [0.0, 0.6, 6.0])
+@pytest.mark.parametrize("distance", [5.0, 60.0, 90.0, 400.0])
+def test_single_tree_rays_that_miss_keep_their_distance(emu, distance, wind):
+    """Beyond the tight boxes' line the pruning distance holds a slack; a ray
+    that enters the root's box and meets nothing returns the distance it came
+    with (the ground's, or the sky's), not one with the slack added."""
+    s = Scene(emu, FAR_SCENE)
+    rays = rays_at((0.0, 1.0, 0.0), 1.0, distance, 128, 4)
+    rays[::2, 6] = distance + 30.0
+    got, want, _ = s.both(rays, wind=wind)
+    assert (want[:, 1] < 0).sum() >= 20 and (want[:, 1] >= 0).sum() >= 10
+    same(got, want)
