@@ -101,7 +101,7 @@ __device__ __forceinline__ void block_classify(const TraceCtx& c, const Ray& r, 
     if (k < nq && open) {
       if (b.res[q] < 0.0f) cls = 2;
     } else if (k < nq) {
-      const int slot = b.slot[q];
+      const int slot = b.slot[q] & (kCapacity - 1);  // (a leaf's slot always is one; no load leaves Order whatever it holds)
       const float* nodes = scene_nodes(c, r.species);
       const float4 lo = ldg4(nodes, 2 * (kCapacity + slot)), hi = ldg4(nodes, 2 * (kCapacity + slot) + 1);
       const uint32_t uid = __ldg(scene_order(c, r.species) + slot);

@@ -38,6 +38,9 @@ enum RayPhase : int { kPhDDA = 0, kPhTree = 1, kPhDone = 3, kPhIdle = 4, kPhBloc
 // such a tree is traversed for real hits alone, and finish_tree looks that
 // first candidate up (first_leaf) if there was none.
 constexpr int kMissCounts = -2;
+// A tree that the batch does not traverse: finish_tree traces it in a fixed
+// order (tree_in_order).
+constexpr int kInOrder = -3;
 
 constexpr int kThreads = 256;  // threads of a block batch (blockbatch.cuh)
 
@@ -58,7 +61,7 @@ struct Ray {
   uint32_t near;    // per axis a bit: the near plane is the box's hi plane
   int boxes;        // the stored boxes in use: 0 the tight ones, kNodeBoxes those of Nodes
   float lbest, lsc; // lbest prunes the traversal: the nearest t so far, or its box entry where that lies beyond it, plus the slack
-  int lfound;       // its leaf slot, -1, or kMissCounts
+  int lfound;       // its leaf slot, -1, kMissCounts or kInOrder
   int group, depth; // nodes 4 group .. 4 group + 3 are tested next; depth 0-7 (nodes at heap level 2 depth + 1)
   uint32_t pending; // deferred nodes per depth, 4 bits each
   int phase;
@@ -104,7 +107,8 @@ __device__ __forceinline__ float box_half(uint32_t pair, uint32_t sel) { return 
 
 // Tree entry with the reference's root test (Arbor.cu:221-223) on the local
 // ray (lro, lrd); keeps the local ray in the batch.  Returns true when the
-// root is accepted and traversal starts.
+// root is accepted and traversal starts (or, with lfound kInOrder, the tree is
+// to be traced in order).
 template <class WB>
 __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int lane, f3 lro, f3 lrd, float lcone, float ltime) {
   r.lfound = -1;
@@ -150,6 +154,16 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
     origin = mk(__ldg(grid), __ldg(grid + 1), __ldg(grid + 2)) - step * kHalfBias;
     m += 4.0f * fmaxf(step.x, fmaxf(step.y, step.z));
   }
+  // Nodes without primitives (0 and 1 among them, no one's children) are stored
+  // inside out over the whole grid, and a margin of half the grid's widest side
+  // turns them right side out: accepted, a walk from nodes 0 or 1 ends at slots
+  // before Order's first.  Twice that distance is kept, for the rounding of the
+  // planes (the margin holds 1e-6 of the distance, so the side is then above
+  // 4e-6 of it and one plane is off by less than 3e-7).  What is smaller beside
+  // its margin - a pebble of 9 cm at 45 m, a leaf alone in a storm - is a few
+  // pixels or a few primitives.  (Also false where the ray is not finite.)
+  const f3 side = xyz(hi) - xyz(lo);
+  if (!(fmaxf(side.x, fmaxf(side.y, side.z)) > 4.0f * m)) r.lfound = kInOrder;
   const f3 oa = (lro + mk(m, m, m) - origin) * linv, ob = (lro - mk(m, m, m) - origin) * linv;
   const bool px = linv.x >= 0.0f, py = linv.y >= 0.0f, pz = linv.z >= 0.0f;
   r.inv = step * linv;
@@ -328,7 +342,7 @@ __device__ __forceinline__ void finish_tree(const TraceCtx& c, Ray& r, WB& b, in
     r.lbest = b.nearest[lane];  // (in place of the traversal's, which holds the slack)
     // The hit comes before its own box, and another one before that box too:
     // which of them a traversal keeps depends on its order.
-    if (r.lfound >= 0 && b.entry[lane] > r.lbest && b.second[lane] <= b.entry[lane]) {
+    if (r.lfound == kInOrder || (r.lfound >= 0 && b.entry[lane] > r.lbest && b.second[lane] <= b.entry[lane])) {
       const TreeResult h = tree_in_order(scene_P(c, r.species), scene_nodes(c, r.species), scene_order(c, r.species), b.rayO[lane], b.rayD[lane],
                                          xyz(b.rayI[lane]), c.wind, r.best / r.lsc, c.refine, WB::kOrdered);
       r.lbest = h.t;
@@ -418,7 +432,7 @@ __device__ __forceinline__ void dda_step(const TraceCtx& c, Ray& r, WB& b, int l
   LocalRay l;
   if (!dda_next(c, r, l)) return;
   if (enter_tree(c, r, b, lane, l.ro, l.rd, l.cone, l.time))
-    r.phase = kPhTree;
+    r.phase = r.lfound == kInOrder ? kPhTreeEnd : kPhTree;
   else
     fold_tree(c, r);  // root rejected: traceTree returns (best, -1)
 }

@@ -124,3 +124,56 @@ def test_single_tree_rays_that_miss_keep_their_distance(emu, distance, wind):
     got, want, _ = s.both(rays, wind=wind)
     assert (want[:, 1] < 0).sum() >= 20 and (want[:, 1] >= 0).sum() >= 10
     same(got, want)
+
+
+SMALL = {
+    "stone of 1 cm at 5 m": ([stone(0.3, 0.5, -0.2, 0.005)], 5.0, 0.004),
+    "stone of 9 cm at 45 m": ([stone(0.3, 0.5, -0.2, 0.045)], 45.0, 0.04),
+    "stone of 12 cm at 60 m": ([stone(0.3, 0.5, -0.2, 0.06)], 60.0, 0.05),
+    "four stones at 35 m": ([stone(0.03 * k, 0.5, 0.02 * k, 0.02) for k in range(4)], 35.0, 0.05),
+    "twig and leaf at 75 m": ([wood((0.0, 0.5, 0.0), (0.0, 0.6, 0.0), 0.02, 0.01), leaf(0.0, 0.6, 0.0, 0.1, 0.04)], 75.0, 0.05),
+}
+
+
+@pytest.mark.parametrize("name", list(SMALL))
+@pytest.mark.parametrize("refine", [True, False])
+def test_small_scene_far_away(emu, name, refine):
+    """The margin by which the boxes are widened is as large as the scene."""
+    records, distance, spread = SMALL[name]
+    s = Scene(emu, records)
+    got, want, _ = s.both(rays_at(records[0][0:3], spread, distance, 96, 1), refine=refine)
+    assert (want[:, 1] >= 0).sum() >= 10
+    same(got, want)
+
+
+@pytest.mark.parametrize("wind", [0.6, 7.0, 40.0])
+def test_one_leaf_in_the_wind(emu, wind):
+    """A shadow segment's margin with the leaf's swing: wider than the scene."""
+    s = Scene(emu, [leaf(0.0, 1.0, 0.0, 0.15, 0.07)])
+    got, want, _ = s.both(rays_at((0.1, 1.0, 0.0), 0.05, 20.0, 96, 2, best=36.0), wind=wind, refine=False)
+    assert (want[:, 1] >= 0).sum() >= 10
+    same(got, want)
+
+
+def test_small_scene_in_a_forest(emu):
+    inst = np.zeros(324 * emu.emu_instance_bytes(), np.uint8)
+    emu.emu_instances(7, _p(inst))
+    s = Scene(emu, [stone(0.2, 1.0, -0.1, 0.05), leaf(0.3, 1.2, 0.0, 0.1, 0.04)])
+    f = inst.view(np.float32).reshape(324, -1)
+    rays = [rays_at((f[t, 0], 1.0, f[t, 1]), 0.4, d, 64, t) for t, d in ((150, 12.0), (171, 40.0), (40, 70.0), (300, 25.0))]
+    for refine in (True, False):
+        got, want, _ = s.both(np.concatenate(rays), inst=inst, refine=refine, wind=0.6)
+        assert (want[:, 1] >= 0).sum() >= 4
+        same(got, want)
+
+
+def test_rays_that_are_not_finite(emu):
+    """Origins and directions with infinities and NaN: no load leaves the
+    scene's buffers (what such a ray hits is not defined)."""
+    s = Scene(emu, [stone(0.3, 0.5, -0.2, 0.045), leaf(0.0, 1.0, 0.0, 0.15, 0.07)])
+    rays = rays_at((0.3, 0.5, -0.2), 0.05, 5.0, 64, 3)
+    bad = [np.nan, np.inf, -np.inf, 1.0e30, 3.0e38]
+    for k in range(60):
+        rays[k, k % 6] = bad[k % 5]
+    s.both(rays)
+    s.both(rays, refine=False)
