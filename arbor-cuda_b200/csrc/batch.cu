@@ -97,7 +97,34 @@ __global__ void __launch_bounds__(kBlock) batch_setup_kernel(const float* __rest
 }
 
 // tracePixels (kShadow false) or the shadow segments of shadePixels (true,
-// visibility into Linear) of every listed view.  Each CTA walks the views in
+// visibility into Linear) of view v, by one CTA.
+template <bool kShadow, class BB>
+__device__ __forceinline__ void batch_view(const BatchView* __restrict__ views, const Camera* __restrict__ cams, const Instance* __restrict__ insts,
+                                           int v, int* __restrict__ queues, const TightView& tight, BB& b) {
+  const Camera& cam = cams[v];
+  const BatchView view = views[v];
+  const int bx = (view.width + 7) / 8;
+  const ViewPool pool{queues + v, view.width, view.height, bx, bx * ((view.height + 3) / 4)};
+  Ray r;
+  if (kShadow) {
+    const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, tight, 0.0001f, cam.time, cam.wind, false, true};
+    ShadowPolicy policy{&c, &cam, view.Hit, view.Linear, view.width, view.height, 0, 0};
+    block_drive(c, r, b, policy, pool);
+  } else {
+    const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, tight, cam.c14 / (float)view.height, cam.time, cam.wind, true, true};
+    PrimaryPolicy policy{&cam, view.Hit, view.width, view.height, 0};
+    block_drive(c, r, b, policy, pool);
+  }
+}
+// The same in a fixed order, for a scene whose Nodes the caller has changed
+// (arbor_batch_view_buffers).
+template <bool kShadow, int Q>
+__device__ __noinline__ void batch_view_in_order(const BatchView* __restrict__ views, const Camera* __restrict__ cams,
+                                                 const Instance* __restrict__ insts, int v, int* __restrict__ queues, OrderBatchOf<Q>* b) {
+  batch_view<kShadow>(views, cams, insts, v, queues, TightView{nullptr, false, 0.0f, 0.0f}, *b);
+}
+
+// The pass over every listed view.  Each CTA walks the views in
 // order and joins each one's pixel queue; its lanes take the view's next
 // pixels as their rays finish, so all CTAs share a view's work.  The view's camera and instance table are read from
 // global memory (the values setup wrote).
@@ -106,26 +133,23 @@ __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* 
                                                                const Instance* __restrict__ insts, const int* __restrict__ list, int n_list,
                                                                int* __restrict__ queues) {
   using BB = BlockBatchOf<Q>;
+  static_assert(sizeof(OrderBatchOf<Q>) <= sizeof(BB), "in the other batch's memory");
   extern __shared__ float4 batch_smem[];
-  BB& b = *reinterpret_cast<BB*>(batch_smem);
+  bool rest = false;  // (the changed scenes' views in a loop of their own: with the call in this one it ran 5 % slower)
   for (int i = 0; i < n_list; i++) {
     const int v = __ldg(list + i);
     const Camera& cam = cams[v];
     if (kShadow && !(cam.shadows > 0.5f)) continue;
-    const BatchView view = views[v];
-    const int bx = (view.width + 7) / 8;
-    const ViewPool pool{queues + v, view.width, view.height, bx, bx * ((view.height + 3) / 4)};
-    const TightView tight = tight_view_warp(view.T, cam.wind);
-    Ray r;
-    if (kShadow) {
-      const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, tight, 0.0001f, cam.time, cam.wind, false, true};
-      ShadowPolicy policy{&c, &cam, view.Hit, view.Linear, view.width, view.height, 0, 0};
-      block_run_pool(c, r, b, policy, pool);
-    } else {
-      const TraceCtx c{view.P, view.Nodes, view.Order, insts + (size_t)v * kForest, tight, cam.c14 / (float)view.height, cam.time, cam.wind, true, true};
-      PrimaryPolicy policy{&cam, view.Hit, view.width, view.height, 0};
-      block_run_pool(c, r, b, policy, pool);
-    }
+    const TightView tight = tight_view_warp(views[v].T, cam.wind);  // uniform
+    if (tight.regular)
+      batch_view<kShadow>(views, cams, insts, v, queues, tight, *reinterpret_cast<BB*>(batch_smem));
+    else
+      rest = true;
+  }
+  for (int i = 0; rest && i < n_list; i++) {
+    const int v = __ldg(list + i);
+    if ((!kShadow || cams[v].shadows > 0.5f) && !tight_view_warp(views[v].T, 0.0f).regular)
+      batch_view_in_order<kShadow>(views, cams, insts, v, queues, reinterpret_cast<OrderBatchOf<Q>*>(batch_smem));
   }
 }
 

@@ -32,7 +32,7 @@
 // finish_tree notices and repeats that tree in a fixed order.  The DDA advance
 // and tree hand-over wait for all results, so they use the reference's best.
 #pragma once
-#include "tracer.cuh"
+#include "orderbatch.cuh"
 
 namespace arbor {
 
@@ -41,7 +41,6 @@ constexpr int kOrderedChunk = 16;  // tree_in_order's chunk of the single-image 
 constexpr int kSlice = 4;        // passes of an advance between two rounds of tests ...
 constexpr int kTreeRun = 8;      // ... of at most this many tree steps each
 constexpr int kMarchRun = 8;     // steps of an SDF march per round
-constexpr int kSolves = 256;     // Newton solves a block keeps for compaction
 
 // Per-block shared-memory batch; Ordered: tree_in_order's chunk.
 template <int Ordered>
@@ -49,6 +48,8 @@ struct BlockBatchOf {
   static constexpr int kQ = kQueue;
   static constexpr int kJobs = kThreads * kQueue;
   static constexpr int kOrdered = Ordered;
+  static constexpr int kRun = kTreeRun;
+  static constexpr bool kWhole = false;
   float4 rayO[kThreads];           // each lane's local ray: origin and wind time
   float4 rayD[kThreads];           // direction and footprint cone
   float4 rayI[kThreads];           // inverse direction and, during the tests, Ray::lbest
@@ -67,6 +68,7 @@ struct BlockBatchOf {
   uint8_t steps[kJobs];            // steps its march has taken
   int solves, unit;                // Newton solves queued and units of tests taken in this round
   uint8_t rayS[kThreads];          // scene (forest of several species)
+  __device__ __forceinline__ int record(const uint32_t*, int q) const { return prim[q]; }
 };
 using BlockBatch = BlockBatchOf<kOrderedChunk>;
 
@@ -76,13 +78,27 @@ __device__ __forceinline__ float candidate_footprint(const BB& b, int q) {
   return fmaxf(0.000005f, b.rayD[q % kThreads].w * fmaxf(0.05f, b.span[q]));
 }
 
-// Resolve this lane's queued leaf slots: the reference's own test of its box
-// in Nodes (Arbor.cu:223) against the nearest t at the tree's entry, its
-// record and its test: a leaf clip, another test (wood, stones, unused
-// records) or none (box not accepted, or an Order entry past the records, not
-// read); appends the tests to the block's job lists.  `open`: the queue was
-// resolved before and only its unfinished marches go on.  The warp's lanes call
-// it together.
+// The test of this lane's queue place q: the reference's own test of its box
+// in Nodes (Arbor.cu:223) against the nearest t at the tree's entry (best0),
+// then its record: 1 a leaf clip, 2 another test (wood, stones, unused records),
+// 0 none (box not accepted, or an Order entry past the records, not read).
+template <int Ordered>
+__device__ __forceinline__ int classify_candidate(const TraceCtx& c, const Ray& r, BlockBatchOf<Ordered>& b, int q, f3 o, f3 inv, float best0) {
+  const int slot = b.slot[q] & (kCapacity - 1);  // (a leaf's slot always is one; no load leaves Order whatever it holds)
+  const float* nodes = scene_nodes(c, r.species);
+  const float4 lo = ldg4(nodes, 2 * (kCapacity + slot)), hi = ldg4(nodes, 2 * (kCapacity + slot) + 1);
+  const uint32_t uid = __ldg(scene_order(c, r.species) + slot);
+  int cls = 0;
+  float spanx;
+  if (node_accept(lo, hi, o, inv, best0, spanx) && uid < (uint32_t)kCapacity)
+    cls = (int)ldg4(scene_P(c, r.species), (int)uid * 6).w == 1 ? 1 : 2;
+  b.prim[q] = (short)uid;
+  b.span[q] = spanx;
+  return cls;
+}
+// Resolve this lane's queued leaf slots and append their tests to the block's
+// job lists.  `open`: the queue was resolved before and only its unfinished
+// marches go on.  The warp's lanes call it together.
 template <class BB>
 __device__ __forceinline__ void block_classify(const TraceCtx& c, const Ray& r, BB& b, int (&count)[2], int nq, bool open) {
   const unsigned full = 0xffffffffu;
@@ -101,15 +117,7 @@ __device__ __forceinline__ void block_classify(const TraceCtx& c, const Ray& r, 
     if (k < nq && open) {
       if (b.res[q] < 0.0f) cls = 2;
     } else if (k < nq) {
-      const int slot = b.slot[q] & (kCapacity - 1);  // (a leaf's slot always is one; no load leaves Order whatever it holds)
-      const float* nodes = scene_nodes(c, r.species);
-      const float4 lo = ldg4(nodes, 2 * (kCapacity + slot)), hi = ldg4(nodes, 2 * (kCapacity + slot) + 1);
-      const uint32_t uid = __ldg(scene_order(c, r.species) + slot);
-      float spanx;
-      if (node_accept(lo, hi, xyz(o), xyz(inv), best0, spanx) && uid < (uint32_t)kCapacity)
-        cls = (int)ldg4(scene_P(c, r.species), (int)uid * 6).w == 1 ? 1 : 2;
-      b.prim[q] = (short)uid;
-      b.span[q] = spanx;
+      cls = classify_candidate(c, r, b, q, xyz(o), xyz(inv), best0);
       b.res[q] = kFar;
       if (c.refine) b.steps[q] = 0;
     }
@@ -129,7 +137,8 @@ __device__ __forceinline__ void block_classify(const TraceCtx& c, const Ray& r, 
 // Newton solve of candidate q, whose clip `ls` passed.
 template <class BB>
 __device__ __forceinline__ void block_solve(const TraceCtx& c, BB& b, int q, const LeafSolve& ls) {
-  b.res[q] = leaf_newton(ls, leaf_shape(scene_P(c, c.species ? b.rayS[q % kThreads] : 0), b.prim[q]), b.res[q], candidate_footprint(b, q));
+  const int s = c.species ? b.rayS[q % kThreads] : 0;
+  b.res[q] = leaf_newton(ls, leaf_shape(scene_P(c, s), b.record(scene_order(c, s), q)), b.res[q], candidate_footprint(b, q));
 }
 
 // Run the block's queued tests: n_leaf leaf clips, n_other others.  Warps take
@@ -151,10 +160,10 @@ __device__ __forceinline__ void block_tests(const TraceCtx& c, BB& b, int n_leaf
     if (u < other_units) {
       const int j = 32 * u + lane;
       if (j < n_other) {
-        const int q = b.job[BB::kJobs - 1 - j], owner = q % kThreads;
+        const int q = b.job[BB::kJobs - 1 - j], owner = q % kThreads, s = c.species ? b.rayS[owner] : 0;
         const float4 o = b.rayO[owner], d = b.rayD[owner];
         int steps = c.refine ? b.steps[q] : 0;
-        b.res[q] = other_t(scene_P(c, c.species ? b.rayS[owner] : 0), b.prim[q], xyz(o), xyz(d), candidate_footprint(b, q), c.refine,
+        b.res[q] = other_t(scene_P(c, s), b.record(scene_order(c, s), q), xyz(o), xyz(d), candidate_footprint(b, q), c.refine,
                            b.rayI[owner].w, -b.res[q], steps, n_other + n_leaf <= 64 ? 64 : kMarchRun);
         if (c.refine) b.steps[q] = (uint8_t)steps;
       }
@@ -165,10 +174,10 @@ __device__ __forceinline__ void block_tests(const TraceCtx& c, BB& b, int n_leaf
       int q = 0;
       if (j < n_leaf) {
         q = b.job[j];
-        const int owner = q % kThreads;
+        const int owner = q % kThreads, s = c.species ? b.rayS[owner] : 0;
         const float4 o = b.rayO[owner], d = b.rayD[owner];
         float tube;
-        solve = leaf_clip(scene_P(c, c.species ? b.rayS[owner] : 0), b.prim[q], xyz(o), xyz(d), o.w, c.wind, ls, tube);
+        solve = leaf_clip(scene_P(c, s), b.record(scene_order(c, s), q), xyz(o), xyz(d), o.w, c.wind, ls, tube);
         // The solve stays inside its clipped interval: one that begins beyond
         // the owner's lbest can neither beat it nor matter to the order.
         solve = solve && !(ls.spanx > b.rayI[owner].w);
@@ -192,24 +201,24 @@ __device__ __forceinline__ void block_tests(const TraceCtx& c, BB& b, int n_leaf
   if (queued > kSolves) {  // uniform; rare: more clips passed than there is room for
     for (int j = tid; j < n_leaf; j += kThreads) {
       if (!(b.job[j] & 0x4000)) continue;
-      const int q = b.job[j] & 0x3fff, owner = q % kThreads;
+      const int q = b.job[j] & 0x3fff, owner = q % kThreads, s = c.species ? b.rayS[owner] : 0;
       const float4 o = b.rayO[owner], d = b.rayD[owner];
       LeafSolve ls;
       float tube;
-      if (leaf_clip_again(scene_P(c, c.species ? b.rayS[owner] : 0), b.prim[q], xyz(o), xyz(d), o.w, c.wind, ls, tube)) block_solve(c, b, q, ls);
+      if (leaf_clip_again(scene_P(c, s), b.record(scene_order(c, s), q), xyz(o), xyz(d), o.w, c.wind, ls, tube)) block_solve(c, b, q, ls);
     }
   }
   __syncthreads();
 }
-static_assert(kThreads * kQueue <= 0x4000, "a queue place fits 14 bits");
+static_assert(kThreads * kQueue <= 0x4000 && kThreads * kMaxChunk <= 0x4000, "a queue place fits 14 bits");
 
 // Apply a lane's results.  A nearer hit replaces the best; an exactly equal
 // one replaces it when the reference meets it first, so the kept primitive
 // does not depend on the order of visits or tests.  The best hit's box entry
 // and the second nearest t tell finish_tree whether the order could matter
 // after all; for that every candidate up to the entry is still tested.
-template <class BB>
-__device__ __forceinline__ void block_apply(const TraceCtx& c, Ray& r, BB& b, int nq) {
+template <int Ordered>
+__device__ __forceinline__ void block_apply(const TraceCtx& c, Ray& r, BlockBatchOf<Ordered>& b, int nq) {
   const int tid = threadIdx.x;
   float best = b.nearest[tid], second = b.second[tid], entry = b.entry[tid];
   for (int k = 0; k < nq; k++) {
@@ -304,24 +313,9 @@ __device__ __forceinline__ bool pool_take(const ViewPool& pool, unsigned idle, i
 // idle.  Every thread of the block calls it; it begins and ends with a
 // barrier.
 template <class BB, class Policy, class Pool>
-__device__ __forceinline__ void block_run_pool(const TraceCtx& c, Ray& r, BB& b, Policy& policy, const Pool& pool) {
+__device__ __forceinline__ void block_drive(const TraceCtx& c, Ray& r, BB& b, Policy& policy, const Pool& pool) {
   const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31;
-  if (!c.tight.regular) {  // uniform in the block
-    bool past = false;
-    while (!past) {
-      int x = 0, y = 0;
-      r.phase = kPhIdle;
-      if (pool_take(pool, full, lane, x, y, past)) policy.start(c, r, x, y);
-      while (r.phase != kPhIdle) {
-        if (r.phase == kPhDDA) dda_step_ordered(c, r, BB::kOrdered);
-        if (r.phase == kPhDone) policy.done(r);
-      }
-      __syncwarp();
-    }
-    __syncthreads();
-    return;
-  }
   int nq = 0;
   bool open = false;     // a march of this lane's queue is unfinished: the lane waits
   bool drained = false;  // uniform in the warp
@@ -344,7 +338,7 @@ __device__ __forceinline__ void block_run_pool(const TraceCtx& c, Ray& r, BB& b,
       }
       // Tree steps a few at a time, so that the cells and tree entries between
       // them, as many instructions each, run for more lanes at once.
-      for (int k = 0; k < kTreeRun; k++) {
+      for (int k = 0; k < BB::kRun; k++) {
         const bool go = r.phase == kPhTree && !open;
         if (!__any_sync(full, go)) break;
         if (go) tree_step(c, r, b, tid, nq);
@@ -353,23 +347,45 @@ __device__ __forceinline__ void block_run_pool(const TraceCtx& c, Ray& r, BB& b,
       if (r.phase == kPhDDA) dda_step(c, r, b, tid);
       if (r.phase == kPhDone) policy.done(r);
     }
-    block_classify(c, r, b, b.count[round], nq, open);
+    // (in a fixed order a chunk is tested whole)
+    const int now = BB::kWhole && r.phase == kPhTree ? 0 : nq;
+    block_classify(c, r, b, b.count[round], now, open);
     if (!__syncthreads_or(r.phase != kPhIdle || !drained)) break;
     const int n_leaf = b.count[round][0], n_other = b.count[round][1];
     if (tid < 2) b.count[round ^ 1][tid] = 0;
     block_tests(c, b, n_leaf, n_other);
     if (tid == 0) b.solves = b.unit = 0;
-    if (nq > 0) {
+    if (now > 0) {
       open = false;
       if (c.refine)
-        for (int k = 0; k < nq; k++) open |= b.res[k * kThreads + tid] < 0.0f;
+        for (int k = 0; k < now; k++) open |= b.res[k * kThreads + tid] < 0.0f;
       if (!open) {
-        block_apply(c, r, b, nq);
+        block_apply(c, r, b, now);
         nq = 0;
         if (r.phase == kPhBlocked) tree_pop(r, b, tid, nq);
       }
     }
   }
+}
+// The same in the fixed order of orderbatch.cuh, out of line: its code and
+// registers stay away from the other loop's.
+template <class BB, class Policy, class Pool>
+__device__ __noinline__ void block_drive_in_order(TraceCtx c, BB* b, Policy policy, Pool pool) {
+  policy.bind(&c);
+  Ray r;
+  block_drive(c, r, *b, policy, pool);
+}
+template <class BB, class Policy, class Pool>
+__device__ __forceinline__ void block_run_pool(const TraceCtx& c, Ray& r, BB& b, Policy& policy, const Pool& pool) {
+  if (!c.tight.regular) {  // uniform in the block
+    using OB = OrderBatchOf<BB::kOrdered>;
+    static_assert(sizeof(OB) <= sizeof(BB) && BB::kOrdered <= kMaxChunk, "in the other batch's memory");
+    Policy copy = policy;
+    copy.bind(nullptr);  // (c itself must not leave the registers)
+    block_drive_in_order(c, reinterpret_cast<OB*>(&b), copy, pool);
+    return;
+  }
+  block_drive(c, r, b, policy, pool);
 }
 
 }  // namespace arbor

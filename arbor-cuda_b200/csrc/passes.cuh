@@ -24,6 +24,7 @@ struct PrimaryPolicy {
   const Camera* cam;
   float* Hit;
   int width, height, pixel;
+  __device__ __forceinline__ void bind(const TraceCtx*) {}
   // The primary ray of pixel (x, y) with the ground plane as its initial
   // nearest hit (tracePixels, Arbor.cu:252).
   __device__ __forceinline__ void start(const TraceCtx& c, Ray& r, int x, int y) {
@@ -373,6 +374,7 @@ struct ShadowPolicy {
   int width, height;
   int pixel, seg;
   f3 trans, origin, light;
+  __device__ __forceinline__ void bind(const TraceCtx* c) { ctx = c; }
   __device__ __forceinline__ void start(const TraceCtx& c, Ray& r, int x, int y) {
     pixel = y * width + x;
     if (shadow_ray(*cam, __ldg(reinterpret_cast<const float4*>(Hit) + pixel), x, y, width, height, origin, light)) {
@@ -424,6 +426,7 @@ struct StagedShadowPolicy {
   int width, height;
   int pixel, seg;
   f3 trans, origin, light;
+  __device__ __forceinline__ void bind(const TraceCtx* c) { ctx = c; }
   __device__ __forceinline__ void start(const TraceCtx& c, Ray& r, int x, int y) {
     pixel = y * width + x;
     const float4 o = reinterpret_cast<const float4*>(Vis)[pixel];

@@ -43,6 +43,7 @@ constexpr int kMissCounts = -2;
 constexpr int kInOrder = -3;
 
 constexpr int kThreads = 256;  // threads of a block batch (blockbatch.cuh)
+constexpr int kSolves = 256;   // Newton solves a block keeps for compaction
 
 // A lane's ray.  The local ray of the tree being traversed (origin,
 // direction, its inverse, wind time, footprint cone) is kept in the block
@@ -436,19 +437,6 @@ __device__ __forceinline__ void dda_step(const TraceCtx& c, Ray& r, WB& b, int l
   else
     fold_tree(c, r);  // root rejected: traceTree returns (best, -1)
 }
-// The next tree traced whole in a fixed order (scenes whose Nodes are not
-// regular).
-__device__ __forceinline__ void dda_step_ordered(const TraceCtx& c, Ray& r, int chunk) {
-  LocalRay l;
-  if (!dda_next(c, r, l)) return;
-  const TreeResult h = tree_in_order(scene_P(c, r.species), scene_nodes(c, r.species), scene_order(c, r.species),
-                                     make_float4(l.ro.x, l.ro.y, l.ro.z, l.time), make_float4(l.rd.x, l.rd.y, l.rd.z, l.cone), inv3(l.rd), c.wind,
-                                     r.lbest, c.refine, chunk);
-  r.lbest = h.t;
-  r.lfound = h.slot;
-  fold_tree(c, r);
-}
-
 // Deferred nodes of one lane: per depth the nodes of the path's group after
 // the first in the order of their visits (visit_key), each as its entry distance
 // (rounded down to 30 bits) with its place in the group in the low two bits; rejected

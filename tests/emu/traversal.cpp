@@ -16,6 +16,7 @@ struct RayPolicy {
   const float* rays;
   float* out;
   int n, index;
+  void bind(const TraceCtx*) {}
   void start(const TraceCtx& c, Ray& r, int x, int y) {
     index = y * 8 + x;
     if (index >= n) return;
@@ -79,6 +80,32 @@ long emu_trace(const float* P, const uint32_t* Order, const float* Nodes, const 
     block_run_pool(c, r, batch, policy, pool);
   });
   return emu::bad_loads;
+}
+
+// The same rays one by one, each tree by tree_in_order.
+void emu_in_order(const float* P, const uint32_t* Order, const float* Nodes, const Instance* inst, const float* rays, int n, float cone,
+                  float time, float wind, int refine, float* out) {
+  emu::buffers = {{(const char*)P, (const char*)(P + kCapacity * kPS)},
+                  {(const char*)Order, (const char*)(Order + kCapacity)},
+                  {(const char*)Nodes, (const char*)(Nodes + kNodeCount * 8)}};
+  const TraceCtx c{P, Nodes, Order, inst, {}, cone, time, wind, refine != 0, inst != nullptr};
+  for (int k = 0; k < n; k++) {
+    const float* a = rays + 7 * k;
+    Ray r;
+    ray_begin(c, r, mk(a[0], a[1], a[2]), mk(a[3], a[4], a[5]), a[6]);
+    while (r.phase != kPhDone) {
+      LocalRay l;
+      if (!dda_next(c, r, l)) continue;
+      const TreeResult h = tree_in_order(P, Nodes, Order, make_float4(l.ro.x, l.ro.y, l.ro.z, l.time),
+                                         make_float4(l.rd.x, l.rd.y, l.rd.z, l.cone), inv3(l.rd), wind, r.lbest, c.refine, kOrderedChunk);
+      r.lbest = h.t;
+      r.lfound = h.slot;
+      fold_tree(c, r);
+    }
+    out[3 * k] = r.best;
+    out[3 * k + 1] = r.found;
+    out[3 * k + 2] = (float)r.foundTree;
+  }
 }
 
 // The same rays one by one in the reference's order.

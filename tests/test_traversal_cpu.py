@@ -53,17 +53,18 @@ class Scene:
         self.T = np.zeros(emu.emu_words(), np.uint32)
         assert emu.emu_boxes(_p(self.P), _p(self.Order), _p(self.Nodes), _p(self.T)) == 0
 
-    def both(self, rays, wind=0.0, refine=True, inst=None, cone=1.0e-3, time=3.25):
+    def both(self, rays, wind=0.0, refine=True, inst=None, cone=1.0e-3, time=3.25, against="emu_reference"):
         """(t, id, tree) of every ray from the block batch and from the
-        reference's traversal; checks that no load left the buffers."""
+        reference's traversal (or another); checks that no load left the
+        buffers."""
         rays = np.ascontiguousarray(rays, np.float32)
         n, f = len(rays), ctypes.c_float
         got, want = np.full((n, 3), np.nan, np.float32), np.full((n, 3), np.nan, np.float32)
         regular = ctypes.c_int(-1)
         bad = self.emu.emu_trace(_p(self.P), _p(self.Order), _p(self.Nodes), _p(self.T), _p(inst), _p(rays), n, f(cone), f(time), f(wind),
                                  int(refine), _p(got), ctypes.byref(regular))
-        self.emu.emu_reference(_p(self.P), _p(self.Order), _p(self.Nodes), _p(inst), _p(rays), n, f(cone), f(time), f(wind), int(refine),
-                               _p(want))
+        getattr(self.emu, against)(_p(self.P), _p(self.Order), _p(self.Nodes), _p(inst), _p(rays), n, f(cone), f(time), f(wind), int(refine),
+                                   _p(want))
         assert bad == 0, f"{bad} loads outside the scene's buffers"
         return got, want, regular.value
 
@@ -177,3 +178,45 @@ def test_rays_that_are_not_finite(emu):
         rays[k, k % 6] = bad[k % 5]
     s.both(rays)
     s.both(rays, refine=False)
+
+
+class Grown(Scene):
+    """A grown scene whose Nodes, changed by `change`, are no longer the bounds
+    of its records."""
+
+    def __init__(self, emu, scene, change):
+        self.emu = emu
+        self.P, self.Order, self.Nodes = (np.array(scene[k]).reshape(-1) for k in ("P", "Order", "Nodes"))
+        change(self.Nodes.reshape(NODE_COUNT, 8))
+        self.T = np.zeros(emu.emu_words(), np.uint32)
+        assert emu.emu_boxes(_p(self.P), _p(self.Order), _p(self.Nodes), _p(self.T)) == 0
+
+
+def cut_leaf_boxes(N):
+    N[CAPACITY:, 0:3] += 0.08 * np.random.RandomState(1).random((CAPACITY, 3)).astype(np.float32)
+
+
+def pad_all(N):
+    N[1:, 0:3] -= 0.01
+    N[1:, 4:7] += 0.01
+
+
+def empty_subtree(N):
+    N[65, 3] = 0.0
+
+
+@pytest.mark.parametrize("change", [cut_leaf_boxes, pad_all, empty_subtree])
+@pytest.mark.parametrize("refine", [True, False])
+def test_nodes_that_are_not_the_records_bounds(emu, scenes, change, refine):
+    """The batch in the fixed order against one tree after another in that
+    order (tree_in_order): with the leaves' boxes cut short, most hits lie
+    before their own box and the order decides which one counts."""
+    s = Grown(emu, scenes(7), change)
+    inst = np.zeros(324 * emu.emu_instance_bytes(), np.uint8)
+    emu.emu_instances(7, _p(inst))
+    rays = np.concatenate([rays_at((0.0, 5.5, 0.0), 3.0, 12.0, 400, 1, best=FAR if refine else 36.0), rays_at((0.0, 3.0, 0.0), 2.0, 9.0, 400, 2)])
+    rays[400:600, :3] = (0.3, 4.0, 0.2)  # from inside the crown
+    for forest in (None, inst):
+        got, want, regular = s.both(rays, wind=0.6, refine=refine, inst=forest, against="emu_in_order")
+        assert regular == 0 and (want[:, 1] >= 0).sum() >= 60
+        same(got, want)
