@@ -121,7 +121,7 @@ __device__ __forceinline__ void batch_view(const BatchView* __restrict__ views, 
 template <bool kShadow, int Q>
 __device__ __noinline__ void batch_view_in_order(const BatchView* __restrict__ views, const Camera* __restrict__ cams,
                                                  const Instance* __restrict__ insts, int v, int* __restrict__ queues, OrderBatchOf<Q>* b) {
-  batch_view<kShadow>(views, cams, insts, v, queues, TightView{nullptr, false, 0.0f, 0.0f}, *b);
+  batch_view<kShadow>(views, cams, insts, v, queues, TightView{nullptr, 0.0f, 0.0f}, *b);
 }
 
 // The pass over every listed view.  Each CTA walks the views in
@@ -141,14 +141,14 @@ __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* 
     const Camera& cam = cams[v];
     if (kShadow && !(cam.shadows > 0.5f)) continue;
     const TightView tight = tight_view_warp(views[v].T, cam.wind);  // uniform
-    if (tight.regular)
+    if (tight.T != nullptr)
       batch_view<kShadow>(views, cams, insts, v, queues, tight, *reinterpret_cast<BB*>(batch_smem));
     else
       rest = true;
   }
   for (int i = 0; rest && i < n_list; i++) {
     const int v = __ldg(list + i);
-    if ((!kShadow || cams[v].shadows > 0.5f) && !tight_view_warp(views[v].T, 0.0f).regular)
+    if ((!kShadow || cams[v].shadows > 0.5f) && tight_view_warp(views[v].T, 0.0f).T == nullptr)
       batch_view_in_order<kShadow>(views, cams, insts, v, queues, reinterpret_cast<OrderBatchOf<Q>*>(batch_smem));
   }
 }

@@ -377,7 +377,7 @@ __device__ __noinline__ void block_drive_in_order(TraceCtx c, BB* b, Policy poli
 }
 template <class BB, class Policy, class Pool>
 __device__ __forceinline__ void block_run_pool(const TraceCtx& c, Ray& r, BB& b, Policy& policy, const Pool& pool) {
-  if (!c.tight.regular) {  // uniform in the block
+  if (c.tight.T == nullptr) {  // uniform in the block
     using OB = OrderBatchOf<BB::kOrdered>;
     static_assert(sizeof(OB) <= sizeof(BB) && BB::kOrdered <= kMaxChunk, "in the other batch's memory");
     Policy copy = policy;

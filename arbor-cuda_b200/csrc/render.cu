@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kBlock, 2) trace_pool_kernel(const float* __re
   if (threadIdx.x == 0) next = 0;
   block_setup(C, cam, nullptr, false, nullptr);
   const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, T, 1, smem) : nullptr;
-  const TightView tight = tight_view_block(T, P, Order, Nodes, 1, cam.wind);
+  const TightView tight = tight_view_block(T, 1, cam.wind);
   const TraceCtx c{P, Nodes, Order, inst, tight, cam.c14 / (float)height, cam.time, cam.wind, true, kForestScene};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kBlock, 2) shadow_pool_kernel(const float* __r
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
   stage_shadows(cam, Hit, Linear, Guide, pool);
   const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, T, 1, smem) : nullptr;
-  const TightView tight = tight_view_block(T, P, Order, Nodes, 1, cam.wind);
+  const TightView tight = tight_view_block(T, 1, cam.wind);
   const TraceCtx c{P, Nodes, Order, inst, tight, 0.0001f, cam.time, cam.wind, false, kForestScene};
   staged_shadow_pool(c, smem.batch, Guide, Linear, pool);
 }
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kBlock, 2) trace_species_kernel(const float* _
   for (int t = threadIdx.x; t < kForest; t += blockDim.x) of[t] = map.of[t];
   block_setup(C, cam, nullptr, false, nullptr);
   const Instance* inst = pass_instances(trig, cam.ws, T, n_scenes, smem);
-  const TightView tight = tight_view_block(T, P, Order, Nodes, n_scenes, cam.wind);
+  const TightView tight = tight_view_block(T, n_scenes, cam.wind);
   const TraceCtx c{P, Nodes, Order, inst, tight, cam.c14 / (float)height, cam.time, cam.wind, true, true, true, of};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kBlock, 2) shadow_species_kernel(const float* 
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
   stage_shadows(cam, Hit, Linear, Guide, pool);
   const Instance* inst = pass_instances(trig, cam.ws, T, n_scenes, smem);
-  const TightView tight = tight_view_block(T, P, Order, Nodes, n_scenes, cam.wind);
+  const TightView tight = tight_view_block(T, n_scenes, cam.wind);
   const TraceCtx c{P, Nodes, Order, inst, tight, 0.0001f, cam.time, cam.wind, false, true, true, of};
   staged_shadow_pool(c, smem.batch, Guide, Linear, pool);
 }
@@ -324,7 +324,8 @@ int launch_tight(const float* P, const uint32_t* Order, const float* Nodes, int 
   return check_launch("tight_kernel");
 }
 
-// tracePixels over the boxes T (tight boxes of the scene, or null: Nodes).
+// tracePixels over the boxes T (tight boxes of the scene, or null: Nodes, in a
+// fixed order).
 int launch_trace(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const uint32_t* T, const float* C,
                  float* Hit, int width, int height, cudaStream_t stream) {
   if (!batch_smem_ready(forest ? (const void*)trace_pool_kernel<true> : (const void*)trace_pool_kernel<false>)) return smem_error(name);

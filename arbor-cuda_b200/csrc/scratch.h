@@ -7,8 +7,8 @@ namespace arbor {
 
 // The tight boxes (tight.cuh) of n scenes for one call on `stream`: made by a
 // kernel queued at construction in memory that is freed, in stream order, at
-// destruction.  `boxes` is null - the pass then traverses Nodes, with the same
-// results - during stream capture (an allocation would become part of the
+// destruction.  `boxes` is null - the pass then traverses Nodes in a fixed order
+// (orderbatch.cuh), with the same results - during stream capture (an allocation would become part of the
 // graph and bar a second instantiation), when no memory can be had, and above
 // kTightMaxScenes.  The memory comes from a pool of the library's own, which
 // keeps at most kScratchKeep bytes when nothing uses it; calls on several

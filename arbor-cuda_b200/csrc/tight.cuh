@@ -225,8 +225,7 @@ static_assert(kTightLeaves / 2 == 256, "one thread per node of the widest inner 
 
 // What a pass traverses.
 struct TightView {
-  const uint32_t* T;  // the tight boxes of its scene(s), kTightWords each; null: Nodes
-  bool regular;       // Nodes is what buildBounds makes of P and Order
+  const uint32_t* T;  // the boxes of its scene(s), kTightWords each; null: Nodes, in a fixed order (orderbatch.cuh)
   float rel, abs;     // the boxes' margin: rel x D + abs
 };
 // Largest swing of a leaf under `wind` whose reach is `reach`.
@@ -236,41 +235,25 @@ __device__ __forceinline__ float swing_margin(float wind, float reach) { return 
 __device__ __forceinline__ TightView tight_view_warp(const uint32_t* T, float wind) {
   const int lane = threadIdx.x & 31;
   const float a = __uint_as_float(__ldg(T + kTightReach + lane)), b = __uint_as_float(__ldg(T + kTightReach + 32 + lane));
-  if (__any_sync(0xffffffffu, !(a >= 0.0f) || !(b >= 0.0f))) return {nullptr, false, 0.0f, 0.0f};
+  if (__any_sync(0xffffffffu, !(a >= 0.0f) || !(b >= 0.0f))) return {nullptr, 0.0f, 0.0f};
   const int reach = __reduce_max_sync(0xffffffffu, __float_as_int(fmaxf(a, b)));
-  return {T, true, kTightRel, swing_margin(wind, __int_as_float(reach))};
+  return {T, kTightRel, swing_margin(wind, __int_as_float(reach))};
 }
-// A block: the view of n scenes' tight boxes; T null: of the scenes
-// themselves, whose Nodes the block then looks through (5 MB a scene; passes
-// without scratch are rare).  Every thread calls it.
-__device__ __forceinline__ TightView tight_view_block(const uint32_t* T, const float* __restrict__ P, const uint32_t* __restrict__ Order,
-                                                      const float* __restrict__ Nodes, int n, float wind) {
+// A block: the view of n scenes' boxes T (null: none were made).  Every thread
+// calls it.
+__device__ __forceinline__ TightView tight_view_block(const uint32_t* T, int n, float wind) {
   __shared__ int reach;
+  if (T == nullptr) return {nullptr, 0.0f, 0.0f};
   if (threadIdx.x == 0) reach = 0;
   __syncthreads();
   bool bad = false;
-  if (T == nullptr) {
-    for (int s = 0; s < n; s++) {
-      const float* p = P + (size_t)s * (kCapacity * kPS);
-      const float* nodes = Nodes + (size_t)s * (kNodeCount * 8);
-      for (int k = threadIdx.x; k < kCapacity; k += blockDim.x) {
-        float4 lo, hi;
-        leaf_record(p, __ldg(Order + (size_t)s * kCapacity + k), lo, hi);
-        bad |= !same_box(lo, hi, ldg4(nodes, 2 * (kCapacity + k)), ldg4(nodes, 2 * (kCapacity + k) + 1));
-        if (k == 0) continue;
-        merge(ldg4(nodes, 4 * k), ldg4(nodes, 4 * k + 1), ldg4(nodes, 4 * k + 2), ldg4(nodes, 4 * k + 3), lo, hi);
-        bad |= !same_box(lo, hi, ldg4(nodes, 2 * k), ldg4(nodes, 2 * k + 1));
-      }
-    }
-    return {nullptr, !__syncthreads_or(bad), 0.0f, 0.0f};
-  }
   for (int k = threadIdx.x; k < n * kTightParts; k += blockDim.x) {
     const float r = __uint_as_float(__ldg(T + (size_t)(k / kTightParts) * kTightWords + kTightReach + k % kTightParts));
     bad |= !(r >= 0.0f);
     atomicMax(&reach, __float_as_int(r));
   }
-  if (__syncthreads_or(bad)) return {nullptr, false, 0.0f, 0.0f};
-  return {T, true, kTightRel, swing_margin(wind, __int_as_float(reach))};
+  if (__syncthreads_or(bad)) return {nullptr, 0.0f, 0.0f};
+  return {T, kTightRel, swing_margin(wind, __int_as_float(reach))};
 }
 
 }  // namespace arbor

@@ -11,7 +11,7 @@
 //   DONE  the ray's result is final
 //
 // The cells and the accepted leaves are the reference's; the order of visits
-// is not.  The traversal runs over the tight boxes of tight.cuh (or Nodes)
+// is not.  The traversal runs over the tight boxes of tight.cuh
 // two heap levels at a time: nodes 4g .. 4g + 3, the grandchildren of node g,
 // are contiguous, and testing them together halves the chain of dependent
 // loads and the loop's passes.  Accepted nodes are visited by the nearer
@@ -74,7 +74,7 @@ struct TraceCtx {
   const float* Nodes;
   const uint32_t* Order;
   const Instance* inst;   // forest instance table (the world-seed registry's, or shared memory)
-  TightView tight;        // the boxes the traversal tests
+  TightView tight;        // the boxes the traversal tests; without them it takes those of Nodes (orderbatch.cuh)
   float cone, time, wind;
   bool refine;            // primary rays: wood refined by the SDF march; false for shadow segments
   bool forest;            // false: the single-tree scene (identity instance)
@@ -129,8 +129,7 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
   b.entry[lane] = 0.0f;
   b.second[lane] = kFar;
   // The margin of the box tests: tight.cuh's, plus the rounding of the slab
-  // distances as one multiply-add each (in Nodes too, whose leaves are tested
-  // again exactly).
+  // distances as one multiply-add each.
   const f3 far = max3(mk(fabsf(lo.x - lro.x), fabsf(lo.y - lro.y), fabsf(lo.z - lro.z)), mk(fabsf(hi.x - lro.x), fabsf(hi.y - lro.y), fabsf(hi.z - lro.z)));
   const float d = length3(far);
   float m = c.tight.rel * d + c.tight.abs;
@@ -148,13 +147,10 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
     r.lbest += slack;
   }
   m += 1.0e-6f * (d + fabsf(lro.x) + fabsf(lro.y) + fabsf(lro.z));
-  f3 origin = mk(0.0f, 0.0f, 0.0f), step = mk(1.0f, 1.0f, 1.0f);
-  if (c.tight.T != nullptr) {
-    const float* grid = reinterpret_cast<const float*>(scene_tight(c, r.species)) + kTightGrid;
-    step = mk(__ldg(grid + 3), __ldg(grid + 4), __ldg(grid + 5));
-    origin = mk(__ldg(grid), __ldg(grid + 1), __ldg(grid + 2)) - step * kHalfBias;
-    m += 4.0f * fmaxf(step.x, fmaxf(step.y, step.z));
-  }
+  const float* grid = reinterpret_cast<const float*>(scene_tight(c, r.species)) + kTightGrid;
+  const f3 step = mk(__ldg(grid + 3), __ldg(grid + 4), __ldg(grid + 5));
+  const f3 origin = mk(__ldg(grid), __ldg(grid + 1), __ldg(grid + 2)) - step * kHalfBias;
+  m += 4.0f * fmaxf(step.x, fmaxf(step.y, step.z));
   // Nodes without primitives (0 and 1 among them, no one's children) are stored
   // inside out over the whole grid, and a margin of half the grid's widest side
   // turns them right side out: accepted, a walk from nodes 0 or 1 ends at slots
@@ -504,37 +500,20 @@ __device__ __forceinline__ void tree_step(const TraceCtx& c, Ray& r, WB& b, int 
   const int node = 4 * r.group;
   float tn[4];       // entries
   uint32_t key[4];   // sort keys, 0xffffffff: rejected
-  if (c.tight.T != nullptr) {
-    const uint4* boxes = reinterpret_cast<const uint4*>(scene_tight(c, r.species) + r.boxes) + 3 * r.group;
-    const uint4 w0 = __ldg(boxes), w1 = __ldg(boxes + 1), w2 = __ldg(boxes + 2);
-    const uint32_t w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
-    const uint32_t nx = r.near & 1u ? kHalfHi : kHalfLo, ny = r.near & 2u ? kHalfHi : kHalfLo, nz = r.near & 4u ? kHalfHi : kHalfLo;
-    const uint32_t fx = nx ^ (kHalfLo ^ kHalfHi), fy = ny ^ (kHalfLo ^ kHalfHi), fz = nz ^ (kHalfLo ^ kHalfHi);
+  const uint4* boxes = reinterpret_cast<const uint4*>(scene_tight(c, r.species) + r.boxes) + 3 * r.group;
+  const uint4 w0 = __ldg(boxes), w1 = __ldg(boxes + 1), w2 = __ldg(boxes + 2);
+  const uint32_t w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
+  const uint32_t nx = r.near & 1u ? kHalfHi : kHalfLo, ny = r.near & 2u ? kHalfHi : kHalfLo, nz = r.near & 4u ? kHalfHi : kHalfLo;
+  const uint32_t fx = nx ^ (kHalfLo ^ kHalfHi), fy = ny ^ (kHalfLo ^ kHalfHi), fz = nz ^ (kHalfLo ^ kHalfHi);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float ax = __fmaf_rn(box_half(w[3 * k], nx), r.inv.x, -r.on.x), ay = __fmaf_rn(box_half(w[3 * k + 1], ny), r.inv.y, -r.on.y),
-                  az = __fmaf_rn(box_half(w[3 * k + 2], nz), r.inv.z, -r.on.z);
-      const float bx = __fmaf_rn(box_half(w[3 * k], fx), r.inv.x, -r.of.x), by = __fmaf_rn(box_half(w[3 * k + 1], fy), r.inv.y, -r.of.y),
-                  bz = __fmaf_rn(box_half(w[3 * k + 2], fz), r.inv.z, -r.of.z);
-      const float tf = fminf(bx, fminf(by, bz));
-      tn[k] = fmaxf(fmaxf(ax, ay), fmaxf(az, 0.0001f));
-      key[k] = tn[k] <= fminf(tf, r.lbest) ? visit_key(c.refine, tn[k], tf, k) : 0xffffffffu;
-    }
-  } else {
-    const float* boxes = scene_nodes(c, r.species);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float4 lo = ldg4(boxes, 2 * (node + k)), hi = ldg4(boxes, 2 * (node + k) + 1);
-      const bool px = !(r.near & 1u), py = !(r.near & 2u), pz = !(r.near & 4u);
-      const float ax = __fmaf_rn(px ? lo.x : hi.x, r.inv.x, -r.on.x), ay = __fmaf_rn(py ? lo.y : hi.y, r.inv.y, -r.on.y),
-                  az = __fmaf_rn(pz ? lo.z : hi.z, r.inv.z, -r.on.z);
-      const float bx = __fmaf_rn(px ? hi.x : lo.x, r.inv.x, -r.of.x), by = __fmaf_rn(py ? hi.y : lo.y, r.inv.y, -r.of.y),
-                  bz = __fmaf_rn(pz ? hi.z : lo.z, r.inv.z, -r.of.z);
-      const float tf = fminf(fmaxf(ax, bx), fminf(fmaxf(ay, by), fmaxf(az, bz)));
-      tn[k] = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.0001f));
-      const bool ok = tn[k] <= fminf(tf, r.lbest) && lo.w > 0.0f && (k > 1 || r.depth > 0);
-      key[k] = ok ? visit_key(c.refine, tn[k], tf, k) : 0xffffffffu;
-    }
+  for (int k = 0; k < 4; k++) {
+    const float ax = __fmaf_rn(box_half(w[3 * k], nx), r.inv.x, -r.on.x), ay = __fmaf_rn(box_half(w[3 * k + 1], ny), r.inv.y, -r.on.y),
+                az = __fmaf_rn(box_half(w[3 * k + 2], nz), r.inv.z, -r.on.z);
+    const float bx = __fmaf_rn(box_half(w[3 * k], fx), r.inv.x, -r.of.x), by = __fmaf_rn(box_half(w[3 * k + 1], fy), r.inv.y, -r.of.y),
+                bz = __fmaf_rn(box_half(w[3 * k + 2], fz), r.inv.z, -r.of.z);
+    const float tf = fminf(bx, fminf(by, bz));
+    tn[k] = fmaxf(fmaxf(ax, ay), fmaxf(az, 0.0001f));
+    key[k] = tn[k] <= fminf(tf, r.lbest) ? visit_key(c.refine, tn[k], tf, k) : 0xffffffffu;
   }
   order2(key[0], key[1]);
   order2(key[2], key[3]);

@@ -27,10 +27,11 @@ struct Range {
   const char *begin, *end;
 };
 inline std::vector<Range> buffers;
-inline long bad_loads = 0;
+inline long bad_loads = 0, loads = 0;
 template <class T>
 T load(const T* p) {
   const char* c = reinterpret_cast<const char*>(p);
+  loads++;
   for (const Range& r : buffers)
     if (c >= r.begin && c + sizeof(T) <= r.end) return *p;
   bad_loads++;

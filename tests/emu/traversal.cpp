@@ -43,6 +43,8 @@ void emu_leaf_nodes(const float* P, const uint32_t* Order, float* Nodes) {  // a
   for (int k = kCapacity - 1; k >= 1; k--) merge(n[4 * k], n[4 * k + 1], n[4 * k + 2], n[4 * k + 3], n[2 * k], n[2 * k + 1]);
 }
 
+static long trace_loads;
+long emu_loads() { return trace_loads; }  // of the last emu_trace
 int emu_words() { return kTightWords; }
 
 // The tight boxes of a scene; returns the loads outside P, Order and Nodes.
@@ -65,13 +67,13 @@ long emu_trace(const float* P, const uint32_t* Order, const float* Nodes, const 
                   {(const char*)Order, (const char*)(Order + kCapacity)},
                   {(const char*)Nodes, (const char*)(Nodes + kNodeCount * 8)}};
   if (T) emu::buffers.push_back({(const char*)T, (const char*)(T + kTightWords)});
-  emu::bad_loads = 0;
+  emu::bad_loads = emu::loads = 0;
   static BlockBatch batch;
   static int next;
   next = 0;
   emu::run(kThreads, 0, 1, [&] {
-    const TightView tight = tight_view_block(T, P, Order, Nodes, 1, wind);
-    if (threadIdx.x == 0) *regular = tight.regular;
+    const TightView tight = tight_view_block(T, 1, wind);
+    if (threadIdx.x == 0) *regular = tight.T != nullptr;
     const TraceCtx c{P, Nodes, Order, inst, tight, cone, time, wind, refine != 0, inst != nullptr};
     const int rows = (n + 7) / 8;
     const PixelPool pool{&next, 8, rows, 1, (rows + 3) / 4};
@@ -79,6 +81,7 @@ long emu_trace(const float* P, const uint32_t* Order, const float* Nodes, const 
     Ray r;
     block_run_pool(c, r, batch, policy, pool);
   });
+  trace_loads = emu::loads;
   return emu::bad_loads;
 }
 

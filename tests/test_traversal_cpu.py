@@ -33,7 +33,7 @@ def emu(tmp_path_factory):
     subprocess.run([gxx, "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-I", include, "-I", CSRC,
                     os.path.join(HERE, "emu", "traversal.cpp"), "-o", out], check=True)
     lib = ctypes.CDLL(out)
-    lib.emu_boxes.restype = lib.emu_trace.restype = ctypes.c_long
+    lib.emu_boxes.restype = lib.emu_trace.restype = lib.emu_loads.restype = ctypes.c_long
     return lib
 
 
@@ -220,3 +220,21 @@ def test_nodes_that_are_not_the_records_bounds(emu, scenes, change, refine):
         got, want, regular = s.both(rays, wind=0.6, refine=refine, inst=forest, against="emu_in_order")
         assert regular == 0 and (want[:, 1] >= 0).sum() >= 60
         same(got, want)
+
+
+@pytest.mark.parametrize("refine", [True, False])
+def test_without_boxes(emu, scenes, refine):
+    """A pass without scratch (under stream capture, above the scratch's scene
+    limit): the fixed order, from the rays' own loads - no CTA looks through the
+    scene first."""
+    s = Grown(emu, scenes(7), lambda N: None)
+    s.T = None
+    rays = rays_at((0.0, 5.5, 0.0), 3.0, 12.0, 64, 5, best=FAR if refine else 36.0)
+    got, want, _ = s.both(rays, refine=refine, against="emu_in_order")
+    assert (want[:, 1] >= 0).sum() >= 10
+    same(got, want)
+    rays[:, 3:6] = (0.0, 1.0, 0.0)  # past the tree: its root's two loads a ray, no more
+    rays[:, 0] = 50.0
+    got, want, _ = s.both(rays, refine=refine, against="emu_in_order")
+    same(got, want)
+    assert emu.emu_loads() <= 2 * len(rays)
