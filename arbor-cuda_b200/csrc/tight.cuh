@@ -43,9 +43,9 @@
 //
 // The boxes are used only where Nodes is what buildBounds makes of P and
 // Order (every leaf box equal to the record's, every inner node the union of
-// its children).  What a scene whose Nodes say anything else shows depends on
-// the order of the traversal; it is traced one tree at a time in a fixed order
-// (tree_in_order).
+// its children) and every record's surface lies inside its box
+// (tighten_record).  What any other scene shows depends on the order of the
+// traversal; it is traversed in a fixed one (orderbatch.cuh).
 #pragma once
 #include "arbor_scene.cuh"
 
@@ -97,18 +97,31 @@ __device__ __forceinline__ void add_axis(float c, float a, float b, float& lo, f
   lo += fminf(a * c, b * c);
   hi += fmaxf(a * c, b * c);
 }
-// Shrinks the box (lo, hi) of leaf record `id` to its blade box and petiole
-// in still air and returns the leaf's reach (0: left as it was, the frame is
-// not orthonormal or a size is negative or not finite).
-__device__ __forceinline__ float tighten_leaf(const float* P, int id, float4& lo, float4& hi) {
+// Shrinks the box (lo, hi) in Nodes of a used record `id`, a leaf's to its
+// blade and petiole in still air, and returns the leaf's reach (0: not a leaf).
+// -1: the surface is not known to lie inside the box - a leaf wider than it is
+// long or curled up beyond its cube, a frame that is not orthonormal, a size
+// that is negative or not finite, an unknown type.  A ray can then pass the box
+// in one place and meet the surface in another, and which hit counts depends on
+// the order: the scene is traversed in the fixed one.
+__device__ __forceinline__ float tighten_record(const float* P, int id, float4& lo, float4& hi) {
   const float4 r0 = ldg4(P, id * 6), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2), r3 = ldg4(P, id * 6 + 3), r4 = ldg4(P, id * 6 + 4);
+  const int type = (int)r0.w;
+  if (!(lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z)) return -1.0f;
+  if (type == 0) return r1.w >= 0.0f && r2.w >= 0.0f ? 0.0f : -1.0f;
+  if (type != 1) return type == 2 ? 0.0f : -1.0f;
   const f3 o = xyz(r0), u = xyz(r1), v = xyz(r2), n = xyz(r3);
   const float len = r1.w, width = r2.w, stem = r4.x;
   const float g = fmaxf(fmaxf(fabsf(dot3(u, u) - 1.0f), fmaxf(fabsf(dot3(v, v) - 1.0f), fabsf(dot3(n, n) - 1.0f))),
                         fmaxf(fabsf(dot3(u, v)), fmaxf(fabsf(dot3(u, n)), fabsf(dot3(v, n)))));
   const float x1 = stem + len + 0.002f, w = fmaxf(width, 0.002f) + 0.0005f;
   const float reach = sqrtf(x1 * x1 + w * w + 0.0045f);  // 0.067^2 across
-  if (!(g < 1.0e-4f) || !(len >= 0.0f) || !(stem >= 0.0f) || !(width >= 0.0f) || !(reach < 1.0e3f)) return 0.0f;
+  if (!(g < 1.0e-4f) || !(len >= 0.0f) || !(stem >= 0.0f) || !(width >= 0.0f) || !(reach < 1.0e3f)) return -1.0f;
+  // Across the blade its height (leaf_height for 0 <= q <= 1, |v| <= width: curl,
+  // twist, 9 mm of cupping, the 1.2 mm rib, the solve's tolerance) within the
+  // clip box's -0.035 .. 0.065, and the petiole's radius.
+  const float height = fabsf(r4.y) + 0.62f * fabsf(r4.z) * w + 0.011f;
+  const float z0 = -fminf(height, 0.037f), z1 = fminf(height, 0.067f);
   const float oc[3] = {o.x, o.y, o.z}, uc[3] = {u.x, u.y, u.z}, vc[3] = {v.x, v.y, v.z}, nc[3] = {n.x, n.y, n.z};
   float l[3], h[3];
 #pragma unroll
@@ -118,12 +131,11 @@ __device__ __forceinline__ float tighten_leaf(const float* P, int id, float4& lo
     h[k] = oc[k] + slack;
     add_axis(uc[k], -0.002f, x1, l[k], h[k]);       // blade -0.001 .. len + 0.001 past the stem, petiole radius 0.0011
     add_axis(vc[k], -w, w, l[k], h[k]);
-    add_axis(nc[k], -0.037f, 0.067f, l[k], h[k]);   // blade box -0.035 .. 0.065 (leaf_clip)
+    add_axis(nc[k], z0, z1, l[k], h[k]);
   }
-  const f3 tl = max3(mk(l[0], l[1], l[2]), xyz(lo)), th = min3(mk(h[0], h[1], h[2]), xyz(hi));
-  if (!(tl.x <= th.x) || !(tl.y <= th.y) || !(tl.z <= th.z)) return 0.0f;
-  lo.x = tl.x, lo.y = tl.y, lo.z = tl.z;
-  hi.x = th.x, hi.y = th.y, hi.z = th.z;
+  if (!(l[0] >= lo.x && l[1] >= lo.y && l[2] >= lo.z && h[0] <= hi.x && h[1] <= hi.y && h[2] <= hi.z)) return -1.0f;
+  lo.x = l[0], lo.y = l[1], lo.z = l[2];
+  hi.x = h[0], hi.y = h[1], hi.z = h[2];
   return reach;
 }
 
@@ -165,7 +177,11 @@ __device__ __forceinline__ void tight_build_part(TightPart& s, const float* __re
     float4 lo, hi;
     leaf_record(P, uid, lo, hi);
     bad |= !same_box(lo, hi, nlo, nhi);
-    if (uid < (uint32_t)kCapacity && (int)ldg4(P, (int)uid * 6).w == 1) reach = fmaxf(reach, tighten_leaf(P, (int)uid, lo, hi));
+    if (lo.w > 0.0f) {
+      const float r = tighten_record(P, (int)uid, lo, hi);
+      bad |= !(r >= 0.0f);
+      reach = fmaxf(reach, r);
+    }
     s.lo[k] = lo;
     s.hi[k] = hi;
     store_tight(T, node, g, lo, hi);

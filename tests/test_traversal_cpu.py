@@ -238,3 +238,65 @@ def test_without_boxes(emu, scenes, refine):
     got, want, _ = s.both(rays, refine=refine, against="emu_in_order")
     same(got, want)
     assert emu.emu_loads() <= 2 * len(rays)
+
+
+WIDE = {
+    # half width far above the length: the blade reaches outside the cube that
+    # bounds it in Nodes
+    "wide leaf": [leaf(0.0, 1.0, 0.0, 0.1, 0.9, stem=0.0)],
+    "wide leaf, turned": [leaf(0.0, 1.0, 0.0, 0.1, 0.9, stem=0.0, frame=((0.6, 0.8, 0.0), (0.0, 0.0, 1.0), (-0.8, 0.6, 0.0)))],
+    "curled leaf": [leaf(0.0, 1.0, 0.0, 0.012, 0.01, stem=0.0, curl=0.06, twist=0.0)],
+    "two wide leaves": [leaf(0.0, 1.0, 0.0, 0.1, 0.9, stem=0.0), leaf(0.4, 1.3, 0.2, 0.1, 0.7, stem=0.02, curl=-0.02)],
+}
+
+
+@pytest.mark.parametrize("wind", [0.0, 0.8])
+@pytest.mark.parametrize("name", list(WIDE))
+def test_leaf_that_reaches_outside_its_box(emu, name, wind):
+    """A ray that passes the leaf's box in Nodes and meets the blade outside it
+    has a hit."""
+    s = Scene(emu, WIDE[name])
+    rays = np.concatenate([rays_at((0.0, 1.0, 0.0), r, d, 128, k) for k, (r, d) in enumerate(((0.02, 4.0), (0.08, 4.0), (0.4, 6.0), (0.12, 1.5)))])
+    rays[1::2, 1] -= 2.0 * (rays[1::2, 1] - 1.0) * 0.93  # half of them nearly along the blade
+    v = np.array([0.0, 1.0, 0.0]) + 0.06 * (np.random.RandomState(8).random((len(rays), 3)) - 0.5) - rays[:, :3]
+    rays[1::2, 3:6] = (v / np.linalg.norm(v, axis=1, keepdims=True))[1::2]
+    for refine in (True, False):
+        got, want, _ = s.both(rays, wind=wind, refine=refine, against="emu_in_order")
+        assert (want[:, 1] >= 0).sum() >= 10
+        same(got, want)
+
+
+def test_record_whose_box_is_inside_out(emu):
+    """A stone with a negative half-axis, wood with negative radii: their boxes
+    in Nodes are inside out, and the slab test takes them as they are."""
+    s = Scene(emu, [stone(0.0, 1.0, 0.0, 0.2, -0.2, 0.2), stone(1.0, 1.0, 0.0, 0.2), wood((0.5, 0.5, 0.0), (0.5, 0.9, 0.1), -0.1, -0.1)])
+    for refine in (True, False):
+        got, want, _ = s.both(np.concatenate([rays_at((0.0, 1.0, 0.0), 0.3, 5.0, 128, 1), rays_at((0.6, 0.8, 0.0), 0.5, 5.0, 128, 2)]), refine=refine)
+        assert (want[:, 1] == 0).sum() >= 10
+        same(got, want)
+
+@pytest.mark.parametrize("kind", ["skewed frame", "negative length", "not a number", "unknown type"])
+def test_records_without_a_bound(emu, kind):
+    """Records whose surface their box says nothing about, among sound ones."""
+    odd = leaf(0.0, 1.0, 0.0, 0.15, 0.07)
+    if kind == "skewed frame":
+        odd[4:7] = (0.5, 0.0, 0.0)
+    elif kind == "negative length":
+        odd[7] = -0.1
+    elif kind == "not a number":
+        odd[17] = np.nan
+    else:
+        odd = stone(0.0, 1.0, 0.0, 0.3)
+        odd[3], odd[7] = 3.0, 0.05
+    s = Scene(emu, [odd, stone(0.1, 1.05, 0.1, 0.05), leaf(0.05, 1.1, -0.05, 0.15, 0.07)])
+    for refine in (True, False):
+        got, want, _ = s.both(np.concatenate([rays_at((0.05, 1.0, 0.0), 0.15, 5.0, 192, 1), rays_at((0.1, 1.0, 0.0), 0.1, 3.0, 192, 2)]),
+                              refine=refine, against="emu_in_order")
+        assert (want[:, 1] >= 0).sum() >= 10
+        same(got, want)
+
+
+def test_grown_scenes_keep_their_tight_boxes(emu, scenes):
+    s = Grown(emu, scenes(7), lambda N: None)
+    _, _, regular = s.both(rays_at((0.0, 5.5, 0.0), 3.0, 12.0, 32, 5))
+    assert regular == 1
