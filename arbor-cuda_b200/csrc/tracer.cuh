@@ -334,7 +334,7 @@ template <class WB>
 __device__ __forceinline__ void finish_tree(const TraceCtx& c, Ray& r, WB& b, int lane) {
   if (r.lfound == kMissCounts) {
     r.lfound = first_leaf(scene_nodes(c, r.species), xyz(b.rayO[lane]), xyz(b.rayI[lane]));
-    r.lbest = kFar;
+    r.lbest = r.lfound >= 0 ? kFar : r.best / r.lsc;
   } else {
     r.lbest = b.nearest[lane];  // (in place of the traversal's, which holds the slack)
     // The hit comes before its own box, and another one before that box too:

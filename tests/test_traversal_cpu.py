@@ -300,3 +300,18 @@ def test_grown_scenes_keep_their_tight_boxes(emu, scenes):
     s = Grown(emu, scenes(7), lambda N: None)
     _, _, regular = s.both(rays_at((0.0, 5.5, 0.0), 3.0, 12.0, 32, 5))
     assert regular == 1
+
+
+@pytest.mark.parametrize("distance", [5.0, 90.0])
+def test_ground_beyond_the_farthest_distance(emu, distance):
+    """Rays just below the horizon meet the ground beyond t = 100000.  One that
+    enters the single tree's root and passes every leaf box keeps that distance;
+    one that meets a leaf box and misses the surface has the miss, at 100000
+    (Arbor.cu:226)."""
+    s = Scene(emu, FAR_SCENE)
+    rays = rays_at((0.0, 1.0, 0.0), 1.0, distance, 256, 6)
+    rays[:, 6] = np.linspace(9.0e4, 4.0e5, 256)
+    for wind in (0.0, 6.0):
+        got, want, _ = s.both(rays, wind=wind)
+        assert (want[:, 0] > FAR).sum() >= 20 and ((want[:, 0] == FAR) & (want[:, 1] >= 0)).sum() >= 5
+        same(got, want)
