@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 
 #include "abi_util.h"
+#include "per_device.h"
 #include "tight.cuh"
 
 namespace cg = cooperative_groups;
@@ -436,16 +437,9 @@ int grid_of(int n, int block) { return (n + block - 1) / block; }
 
 // Host helpers reused by the engine and the fused build.
 int launch_sort(uint32_t* Keys, uint32_t* Order, cudaStream_t stream) {
-  static bool ready[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (!ready[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(radix_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-    if (e != cudaSuccess) {
-      set_error("arbor_sortKeys: cannot reserve %zu bytes of shared memory per CTA: %s", sizeof(SortSmem), cudaGetErrorString(e));
-      return ARBOR_ERR_CUDA;
-    }
-    ready[dev] = true;
+  if (!smem_opt_in<radix_sort_kernel>((int)sizeof(SortSmem))) {
+    set_error("arbor_sortKeys: cannot reserve %zu bytes of shared memory per CTA: %s", sizeof(SortSmem), cudaGetErrorString(cudaGetLastError()));
+    return ARBOR_ERR_CUDA;
   }
   radix_sort_kernel<<<kSortCtas, kSortThreads, sizeof(SortSmem), stream>>>(Keys, Order);
   count_launch();

@@ -40,6 +40,7 @@
 
 #include "abi_util.h"
 #include "arbor_math.cuh"
+#include "per_device.h"
 
 namespace arbor {
 namespace {
@@ -1130,13 +1131,8 @@ int launch_conv(const ConvArgs& a, cudaStream_t s) {
   g.y = (unsigned)(a.cout / (nt * 8));
 #define DN_CONV(KC, NT)                                                                                                 \
   do {                                                                                                                  \
-    static bool ready = false;                                                                                          \
-    if (!ready) {                                                                                                       \
-      if (cudaFuncSetAttribute(conv_kernel<KC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem_bytes<KC, NT>()) != \
-          cudaSuccess)                                                                                                  \
-        return cuda_fail("cudaFuncSetAttribute (conv)", cudaGetLastError());                                            \
-      ready = true;                                                                                                     \
-    }                                                                                                                   \
+    if (!smem_opt_in<conv_kernel<KC, NT>>(conv_smem_bytes<KC, NT>()))                                                   \
+      return cuda_fail("cudaFuncSetAttribute (conv)", cudaGetLastError());                                              \
     conv_kernel<KC, NT><<<g, 128, conv_smem_bytes<KC, NT>(), s>>>(a);                                                   \
   } while (0)
   if (kc == 32 && nt == 8) DN_CONV(32, 8);
@@ -1150,11 +1146,6 @@ int launch_conv(const ConvArgs& a, cudaStream_t s) {
   return check_launch("conv_kernel");
 }
 
-int device_sms() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  return sms;
-}
 // Shared memory per CTA is padded so that the CTAs one SM can hold never ask
 // for more than its 512 TMEM columns together (an allocation then never
 // waits on another CTA).
@@ -1168,19 +1159,12 @@ template <int N, int CIN, int S, int B>
 int launch_row(const ConvArgs& a, int* err, cudaStream_t s) {
   constexpr int smem = conv_smem_padded(conv_row_smem_bytes<N, CIN, S, B>(), pow2_cols(B * N));
   static_assert(smem <= 227 * 1024, "shared memory per CTA");
-  static bool ready = false;
-  static int sms = 0;
-  if (!ready) {
-    if (cudaFuncSetAttribute(conv_row_kernel<N, CIN, S, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return cuda_fail("cudaFuncSetAttribute (conv_row)", cudaGetLastError());
-    sms = device_sms();
-    ready = true;
-  }
+  if (!smem_opt_in<conv_row_kernel<N, CIN, S, B>>(smem)) return cuda_fail("cudaFuncSetAttribute (conv_row)", cudaGetLastError());
   const int per_sm = std::max(1, 228 * 1024 / (smem + 1024));
   // One wave: as many row groups per segment as the CTA slots hold (rounded up
   // instead, 150 groups on 148 SMs took two waves and twice the time).
   const long segs = (long)((a.w + 127) / 128) * a.n;
-  const long want = std::max(1L, (long)sms * per_sm / segs);
+  const long want = std::max(1L, (long)device_sms() * per_sm / segs);
   const long rows = std::min<long>(a.h, std::max(4L, (a.h + want - 1) / want));
   const dim3 grid((unsigned)(segs * ((a.h + rows - 1) / rows)));
   conv_row_kernel<N, CIN, S, B><<<grid, kConvThreads, smem, s>>>(a, (int)rows, err);
@@ -1192,17 +1176,10 @@ int launch_tc(const ConvArgs& a, int* err, cudaStream_t s) {
   constexpr int smem = conv_smem_padded(conv_tc_smem_bytes<N, R, S, B>(), pow2_cols(B * R * N));
   static_assert(B * R * N <= 512, "TMEM columns");
   static_assert(smem <= 227 * 1024, "shared memory per CTA");
-  static bool ready = false;
-  static int sms = 0;
-  if (!ready) {
-    if (cudaFuncSetAttribute(conv_tc_kernel<N, R, S, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return cuda_fail("cudaFuncSetAttribute (conv_tc)", cudaGetLastError());
-    sms = device_sms();
-    ready = true;
-  }
+  if (!smem_opt_in<conv_tc_kernel<N, R, S, B>>(smem)) return cuda_fail("cudaFuncSetAttribute (conv_tc)", cudaGetLastError());
   const int per_sm = std::max(1, 228 * 1024 / (smem + 1024));
   const int tiles = (a.w + 127) / 128 * ((a.h + R - 1) / R) * a.n;
-  conv_tc_kernel<N, R, S, B><<<std::min(tiles, sms * per_sm), kConvThreads, smem, s>>>(a, tiles, err);
+  conv_tc_kernel<N, R, S, B><<<std::min(tiles, device_sms() * per_sm), kConvThreads, smem, s>>>(a, tiles, err);
   count_launch();
   return check_launch("conv_tc_kernel");
 }

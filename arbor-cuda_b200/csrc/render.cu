@@ -13,6 +13,7 @@
 
 #include "abi_util.h"
 #include "passes.cuh"
+#include "per_device.h"
 #include "scratch.h"
 
 namespace arbor {
@@ -270,20 +271,9 @@ __global__ void __launch_bounds__(kBlock) shade_inorder_kernel(const float* __re
   reinterpret_cast<float4*>(Guide)[pixel] = make_float4(sh.guide.x, sh.guide.y, sh.guide.z, 1.0f);
 }
 
-// Opt a kernel in to kPassSmemTable of dynamic shared memory, once per device.
-inline bool batch_smem_ready(const void* kernel) {
-  static const void* done[64][8] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  for (int i = 0; i < 8; i++) {
-    if (done[dev][i] == kernel) return true;
-    if (done[dev][i] == nullptr) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmemTable) != cudaSuccess) return false;
-      done[dev][i] = kernel;
-      return true;
-    }
-  }
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmemTable) == cudaSuccess;
+template <auto Kernel>
+bool pass_smem_ready() {
+  return smem_opt_in<Kernel>((int)kPassSmemTable);
 }
 
 dim3 pixel_grid(int w, int h) { return dim3((w + kTile - 1) / kTile, (h + kTile - 1) / kTile); }
@@ -291,12 +281,8 @@ dim3 pixel_grid(int w, int h) { return dim3((w + kTile - 1) / kTile, (h + kTile 
 // Persistent grid: 2 CTAs per SM (the register and shared-memory limit of
 // the batched tracer), or one CTA per 8x4 block when the image has fewer.
 dim3 pool_grid(int w, int h) {
-  static int sms[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (sms[dev] == 0 && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms[dev] = 148;
   const long blocks = (long)((w + 7) / 8) * ((h + 3) / 4);
-  return dim3((unsigned)std::min<long>(blocks, 2L * sms[dev]));
+  return dim3((unsigned)std::min<long>(blocks, 2L * device_sms()));
 }
 // Checks of tracePixels / shadePixels, shared by the entries and the engine.
 int trace_checks(const char* name, const float* P, const float* Nodes, const uint32_t* Order, const float* C, const float* Hit, int width,
@@ -328,7 +314,7 @@ int launch_tight(const float* P, const uint32_t* Order, const float* Nodes, int 
 // fixed order).
 int launch_trace(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const uint32_t* T, const float* C,
                  float* Hit, int width, int height, cudaStream_t stream) {
-  if (!batch_smem_ready(forest ? (const void*)trace_pool_kernel<true> : (const void*)trace_pool_kernel<false>)) return smem_error(name);
+  if (!(forest ? pass_smem_ready<trace_pool_kernel<true>>() : pass_smem_ready<trace_pool_kernel<false>>())) return smem_error(name);
   if (forest)
     trace_pool_kernel<true><<<pool_grid(width, height), kBlock, T ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), T, Hit, width, height);
   else
@@ -342,7 +328,7 @@ int launch_trace(const char* name, bool forest, const float* P, const float* Nod
 // every pixel.
 int launch_shade(const char* name, bool forest, const float* P, const float* Nodes, const uint32_t* Order, const uint32_t* T, const float* C,
                  const float* Hit, float* Linear, float* Guide, float* Normal, int width, int height, cudaStream_t stream) {
-  if (!batch_smem_ready(forest ? (const void*)shadow_pool_kernel<true> : (const void*)shadow_pool_kernel<false>)) return smem_error(name);
+  if (!(forest ? pass_smem_ready<shadow_pool_kernel<true>>() : pass_smem_ready<shadow_pool_kernel<false>>())) return smem_error(name);
   if (forest) {
     shadow_pool_kernel<true><<<pool_grid(width, height), kBlock, T ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), T, Hit, Guide, Linear,
                                                                                        width, height);
@@ -429,7 +415,7 @@ extern "C" int arbor_traceSpeciesPixels(const float* P, const float* Nodes, cons
                        {Hit, empty ? 0 : image_bytes(width, height), true, 16, "Hit"}};
   if (int s = check_bindings(name, b)) return s;
   if (empty) return ARBOR_OK;
-  if (!batch_smem_ready((const void*)trace_species_kernel)) return smem_error(name);
+  if (!pass_smem_ready<trace_species_kernel>()) return smem_error(name);
   const TightScratch t(P, Order, Nodes, n_species, C, false, stream);
   if (t.status) return t.status;
   trace_species_kernel<<<pool_grid(width, height), kBlock, t.boxes ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), t.boxes, n_species, Hit, width,
@@ -451,7 +437,7 @@ extern "C" int arbor_shadeSpeciesPixels(const float* P, const float* Nodes, cons
                        {Guide, img, true, 16, "Guide"}};
   if (int s = check_bindings(name, b)) return s;
   if (empty) return ARBOR_OK;
-  if (!batch_smem_ready((const void*)shadow_species_kernel)) return smem_error(name);
+  if (!pass_smem_ready<shadow_species_kernel>()) return smem_error(name);
   const TightScratch t(P, Order, Nodes, n_species, C, true, stream);
   if (t.status) return t.status;
   shadow_species_kernel<<<pool_grid(width, height), kBlock, t.boxes ? kPassSmem : kPassSmemTable, stream>>>(P, Nodes, Order, C, world_trig(), t.boxes, n_species, Hit, Guide,
