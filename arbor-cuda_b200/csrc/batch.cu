@@ -28,8 +28,8 @@
 //
 // The autotuner times the trace, shadow and compose kernels on a sample of
 // the views for each compose tile shape (16x16 or 32x8), CTAs per SM (1 or
-// 2), view order (as given, or the largest views first) and chunk of
-// order-dependent trees (12 or 16 candidates), and keeps the fastest.
+// 2) and view order (as given, or the largest views first), and keeps the
+// fastest.
 #include <algorithm>
 #include <cstring>
 #include <new>
@@ -638,43 +638,45 @@ extern "C" int arbor_batch_autotune(arbor_batch* b, int sample_views, arbor_batc
   int status = join_user(b), slot = 0;
   float best_ms = -1.0f;
   arbor_batch_config chosen = keep;
+  // The queue (the chunk of a tree whose answer depends on the order) changes
+  // such a tree's answer and not the time, so it is not tuned: the batch keeps
+  // its own, and both table entries of a configuration hold the one time.
   for (int tw : {16, 32})
     for (int ctas : {1, 2})
-      for (int order : {0, 1})
-        for (int q : {12, 16}) {
-          const arbor_batch_config cfg{tw, ctas, order, q};
-          std::vector<int4> t;
-          const std::vector<int> vo = view_order(b, subset, order);
-          trace_tiles(b, vo, tw, t);
-          float ms = 0.0f;
+      for (int order : {0, 1}) {
+        const arbor_batch_config cfg{tw, ctas, order, keep.queue};
+        std::vector<int4> t;
+        const std::vector<int> vo = view_order(b, subset, order);
+        trace_tiles(b, vo, tw, t);
+        float ms = 0.0f;
+        if (status == ARBOR_OK) {
+          // the previous candidate's kernels must be done with the tile list
+          cudaError_t ce = cudaStreamSynchronize(b->own);
+          if (ce == cudaSuccess) ce = cudaMemcpyAsync(b->tiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice, b->own);
+          if (ce == cudaSuccess) ce = cudaMemcpyAsync(b->vlist, vo.data(), vo.size() * sizeof(int), cudaMemcpyHostToDevice, b->own);
+          if (ce != cudaSuccess) status = cuda_fail("autotune tile upload", ce);
+          // one untimed run, then one timed run
+          for (int rep = 0; rep < 2 && status == ARBOR_OK; rep++) {
+            if ((status = launch_setup(b, b->own))) break;
+            if (rep == 1 && (ce = cudaEventRecord(e0, b->own)) != cudaSuccess) status = cuda_fail("cudaEventRecord", ce);
+            if (status || (status = launch_trace_shade(b, cfg, b->tiles, (int)t.size(), (int)vo.size(), b->own))) break;
+            if (rep == 1 && (ce = cudaEventRecord(e1, b->own)) != cudaSuccess) status = cuda_fail("cudaEventRecord", ce);
+          }
           if (status == ARBOR_OK) {
-            // the previous candidate's kernels must be done with the tile list
-            cudaError_t ce = cudaStreamSynchronize(b->own);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(b->tiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice, b->own);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(b->vlist, vo.data(), vo.size() * sizeof(int), cudaMemcpyHostToDevice, b->own);
-            if (ce != cudaSuccess) status = cuda_fail("autotune tile upload", ce);
-            // one untimed run, then one timed run
-            for (int rep = 0; rep < 2 && status == ARBOR_OK; rep++) {
-              if ((status = launch_setup(b, b->own))) break;
-              if (rep == 1 && (ce = cudaEventRecord(e0, b->own)) != cudaSuccess) status = cuda_fail("cudaEventRecord", ce);
-              if (status || (status = launch_trace_shade(b, cfg, b->tiles, (int)t.size(), (int)vo.size(), b->own))) break;
-              if (rep == 1 && (ce = cudaEventRecord(e1, b->own)) != cudaSuccess) status = cuda_fail("cudaEventRecord", ce);
-            }
-            if (status == ARBOR_OK) {
-              if ((ce = cudaEventSynchronize(e1)) != cudaSuccess)
-                status = cuda_fail("cudaEventSynchronize", ce);
-              else
-                cudaEventElapsedTime(&ms, e0, e1);
-            }
-            count_launch(8);  // two runs of setup, trace, shadow, compose
+            if ((ce = cudaEventSynchronize(e1)) != cudaSuccess)
+              status = cuda_fail("cudaEventSynchronize", ce);
+            else
+              cudaEventElapsedTime(&ms, e0, e1);
           }
-          if (ms_table) ms_table[slot] = ms;
-          slot++;
-          if (status == ARBOR_OK && (best_ms < 0.0f || ms < best_ms)) {
-            best_ms = ms;
-            chosen = cfg;
-          }
+          count_launch(8);  // two runs of setup, trace, shadow, compose
         }
+        if (ms_table) ms_table[slot] = ms_table[slot + 1] = ms;
+        slot += 2;
+        if (status == ARBOR_OK && (best_ms < 0.0f || ms < best_ms)) {
+          best_ms = ms;
+          chosen = cfg;
+        }
+      }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (status) {

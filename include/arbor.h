@@ -361,12 +361,13 @@ ARBOR_API int arbor_batch_create(arbor_batch** out, const int* seeds, int n_scen
 ARBOR_API int arbor_batch_set_cameras(arbor_batch* b, const float* C, int n_views);
 ARBOR_API int arbor_batch_configure(arbor_batch* b, const arbor_batch_config* cfg);
 ARBOR_API int arbor_batch_get_config(arbor_batch* b, arbor_batch_config* cfg);
-/* Times the trace, shadow and compose kernels of every configuration (16, ordered by
- * tile_width, ctas_per_sm, order, queue, the last varying fastest) on
- * `sample_views` views spread over the batch (all when <= 0), writes the
- * times to ms_table (nullable, 16 floats), keeps the fastest and returns it
- * in best (nullable).  The sample renders overwrite those views' Hit,
- * Linear and Guide. */
+/* Times the trace, shadow and compose kernels of every tile_width, ctas_per_sm
+ * and order on `sample_views` views spread over the batch (all when <= 0),
+ * keeps the fastest with the batch's own queue and returns it in best
+ * (nullable).  ms_table (nullable, 16 floats) is ordered by tile_width,
+ * ctas_per_sm, order, queue, the last varying fastest; queue does not change
+ * the time, and its two entries are the same.  The sample renders overwrite
+ * those views' Hit, Linear and Guide. */
 ARBOR_API int arbor_batch_autotune(arbor_batch* b, int sample_views, arbor_batch_config* best, float* ms_table);
 /* Renders every view: one graph launch. */
 ARBOR_API int arbor_batch_render(arbor_batch* b);
