@@ -16,15 +16,15 @@
 //   batch_compose_kernel      persistent CTAs pull tiles of every view from
 //                             one global queue: shadePixels' colours
 //                             (Arbor.cu:277-289) with that visibility
-//   batch_filter_kernel       persistent CTAs pull 32x8 tiles and run the
+//   batch_filter_kernel       persistent CTAs pull 32x16 tiles and run the
 //                             fused filterLighting + resolvePixels
 //                             (Arbor.cu:292-304)
 //
 // Every per-pixel value is computed by the same device code as the
 // single-image entries (passes.cuh), so a view renders as
 // arbor_tracePixels + arbor_shadePixels + arbor_filterResolve render it with
-// the same C, apart from the order in which exactly equal hit distances are
-// met (see blockbatch.cuh).
+// the same C, with queue 12 apart from trees whose answer depends on the order
+// (blockbatch.cuh).
 //
 // The autotuner times the trace, shadow and compose kernels on a sample of
 // the views for each compose tile shape (16x16 or 32x8), CTAs per SM (1 or

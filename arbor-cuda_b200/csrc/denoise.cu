@@ -13,15 +13,19 @@
 // are multiples of 16.
 //
 // Kernels:
-//   conv_tc_kernel  the forward 3x3 convolutions on tcgen05 (TMEM
-//                   accumulators), used by inference and training
+//   conv_row_kernel, conv_tc_kernel
+//                   the forward 3x3 convolutions and the backward data pass on
+//                   tcgen05 (TMEM accumulators): rows streamed past resident
+//                   weights, or chunks of input channels
 //   conv_kernel     3x3 convolution as an implicit GEMM: a CTA computes an
 //                   8x8-pixel tile (partial at the image edge) for 16, 32 or
 //                   64 output channels; input halo
 //                   and weights are staged in shared memory 16 or 32 input
-//                   channels at a time.  The same kernel runs the backward
-//                   data pass on rotated, transposed weights, with the
-//                   previous layer's activation derivative in its epilogue.
+//                   channels at a time.  For the 160- and 224-channel data
+//                   passes, and every layer of the mma.sync backend.  The
+//                   backward data pass is the same convolution on rotated,
+//                   transposed weights, with the previous layer's activation
+//                   derivative in its epilogue.
 //   wgrad_kernel    weight gradients: a GEMM over pixels of the output
 //                   gradient and the shifted input; each CTA writes its
 //                   pixel range's partial sums, reduce_kernel adds the
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(128) conv_kernel(ConvArgs a) {
 // ------------------------------------------- tcgen05 convolution (sm_100a) --
 // The same 3x3 convolution on the 5th-generation tensor cores, in two forms of
 // one warp-specialised pipeline.  A CTA works on a 128-pixel column segment:
-// four producer warps copy input rows (130 pixels with the halo) and weights
+// eight producer warps copy input rows (130 pixels with the halo) and weights
 // into shared memory with cp.async, in the K-major, non-swizzled core-matrix
 // layout the MMA reads (8 rows of 16 bytes per core matrix), so that the A
 // operand of an output row and a tap (dy, dx) is a staged row shifted by dx and
@@ -1184,7 +1188,7 @@ int launch_tc(const ConvArgs& a, int* err, cudaStream_t s) {
   return check_launch("conv_tc_kernel");
 }
 
-bool tc_shape(const ConvArgs& a) { return a.cout == 16 || a.cout == 32 || a.cout == 64 || a.cout == 96 || a.cout == 128; }
+bool tc_shape(const ConvArgs& a) { return (a.cout == 16 && a.cin == 32) || a.cout == 32 || a.cout == 64 || a.cout == 96 || a.cout == 128; }
 int launch_conv_tc(const ConvArgs& a, int* err, cudaStream_t s) {
   // The layers whose weights and a ring of rows fit in shared memory stream
   // rows; the others take chunks of 16 input channels.
@@ -1195,7 +1199,6 @@ int launch_conv_tc(const ConvArgs& a, int* err, cudaStream_t s) {
   if (a.cout == 64 && a.cin == 64) return launch_row<64, 64, 6, 8>(a, err, s);
   if (a.cout == 96 && a.cin == 64) return launch_row<96, 64, 5, 5>(a, err, s);
   switch (a.cout) {
-    case 16: return launch_tc<16, 8, 4, 2>(a, err, s);
     case 32: return launch_tc<32, 16, 2, 1>(a, err, s);
     case 64: return launch_tc<64, 8, 3, 1>(a, err, s);
     case 96: return launch_tc<96, 4, 4, 1>(a, err, s);

@@ -199,7 +199,7 @@ __device__ float spec_ggx(f3 n, f3 v, f3 l, float rough) {
 
 // shadePixels (Arbor.cu:277-289) is split at the sun-visibility call:
 // shade_pre computes everything before it, the shadow segments are traced by
-// the warp tracer, shade_post composes the colour.  Each value is computed
+// the block batch, shade_post composes the colour.  Each value is computed
 // with the reference's operations in the reference's order; the colour
 // before haze is (direct * visibility) * (4.8, 4.2, 3.1) + albedo * ambient.
 struct Shading {
@@ -361,7 +361,7 @@ __device__ __forceinline__ bool shadow_ray(const Camera& cam, float4 hit, int x,
   return true;
 }
 
-// Shadow segments alone (Arbor.cu:271-274), for the persistent shadow pass:
+// Shadow segments alone (Arbor.cu:271-274), for the batch's persistent shadow pass:
 // a pixel's visibility toward the sun is written to Vis (the Linear buffer,
 // which the compose pass then overwrites with the colour); pixels without a
 // shadow ray are left alone.
@@ -404,15 +404,6 @@ struct ShadowPolicy {
     r.phase = kPhIdle;
   }
 };
-
-// Shadow segments of every pixel of a persistent CTA's pool.
-template <class WB>
-__device__ __forceinline__ void shadow_pool(const TraceCtx& c, const Camera& cam, WB& b, const float* __restrict__ Hit, float* __restrict__ Vis,
-                                            const PixelPool& pool) {
-  ShadowPolicy policy{&c, &cam, Hit, Vis, pool.width, pool.height, 0, 0};
-  Ray r;
-  block_run_pool(c, r, b, policy, pool);
-}
 
 // The same shadow segments with each pixel's ray staged in memory by the
 // same CTA (stage_shadows): origin in Vis (w = 1 when the pixel has a

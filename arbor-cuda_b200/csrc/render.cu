@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kBlock, 4) shade_compose_species_kernel(const 
 
 // tracePixels and shadePixels with the reference's traversal as written
 // (Arbor.cu:220-289): one ray per thread over 16x16-pixel CTAs, candidates
-// tested in visiting order, children nearest entry first, no warp batching.
+// tested in visiting order, children nearest entry first, no batching.
 // Slower forms kept to check that the batched passes' order does not change
 // a result (the in-order entry points).
 template <bool kForestScene>

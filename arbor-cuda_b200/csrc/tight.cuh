@@ -13,7 +13,7 @@
 //
 // Why no result changes.  A primitive counts only when the ray passes its box
 // in Nodes, and that test is still made, exactly, on every candidate
-// (batch_tests).  The tight boxes only drop candidates whose test returns no
+// (classify_candidate).  The tight boxes only drop candidates whose test returns no
 // hit.  To be sure of that the traversal widens every tight box by a margin m
 // that covers what the FP32 tests can report off the true surface:
 //  - the sphere and cone quadratics cancel: their discriminant is off by at

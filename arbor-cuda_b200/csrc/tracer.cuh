@@ -15,8 +15,9 @@
 // two heap levels at a time: nodes 4g .. 4g + 3, the grandchildren of node g,
 // are contiguous, and testing them together halves the chain of dependent
 // loads and the loop's passes.  Accepted nodes are visited by the nearer
-// midpoint of their span (primary rays) or the nearer entry (shadow segments).  The result is the nearest hit over the
-// accepted leaf boxes whatever the order (blockbatch.cuh gives the argument),
+// midpoint of their span (primary rays) or the nearer entry (shadow segments).
+// The result is the nearest hit over the accepted leaf boxes whatever the order
+// (blockbatch.cuh gives the argument),
 // as long as each hit lies inside its primitive's box; between exactly equal
 // hit distances (leaves sharing a petiole base, wood segments sharing a
 // joint) the one the reference meets first is kept (ref_before).  Where a hit
@@ -135,7 +136,7 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
   float m = c.tight.rel * d + c.tight.abs;
   float slack = 0.0f;
   r.boxes = 0;
-  if (c.refine && m > kTightMost) {  // (a shadow segment's 36 m stay below it)
+  if (c.refine && m > kTightMost) {  // (a shadow segment is 36 m at most; its pruning has no slack)
     // The boxes are not widened, but a hit may still come before its box by
     // the margin: pruning allows for it.
     slack = m;
