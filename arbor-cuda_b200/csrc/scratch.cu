@@ -7,6 +7,16 @@ namespace arbor {
 namespace {
 
 constexpr int kMaxDevices = 64;
+
+// While one lives, this thread's allocations do not disturb a capture that
+// another thread has begun in the global mode (torch's default): a pool that
+// has to grow would invalidate it.
+struct OtherCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  OtherCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OtherCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 
@@ -20,9 +30,6 @@ cudaMemPool_t scratch_pool() {
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = dev;
-  // (another thread's capture on another stream must not be disturbed)
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
   cudaMemPool_t pool = nullptr;
   uint64_t keep = kScratchKeep;
   if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
@@ -33,7 +40,6 @@ cudaMemPool_t scratch_pool() {
     cudaMemPoolDestroy(pool);
     pool = nullptr;
   }
-  cudaThreadExchangeStreamCaptureMode(&mode);
   g_pool[dev] = pool;
   return pool;
 }
@@ -48,6 +54,7 @@ TightScratch::TightScratch(const float* P, const uint32_t* Order, const float* N
     return;
   }
   if (cs != cudaStreamCaptureStatusNone || n_scenes > kTightMaxScenes) return;
+  const OtherCaptures undisturbed;
   const cudaMemPool_t pool = scratch_pool();
   void* p = nullptr;
   if (pool == nullptr || cudaMallocFromPoolAsync(&p, tight_bytes(n_scenes), pool, stream) != cudaSuccess) {
@@ -59,7 +66,9 @@ TightScratch::TightScratch(const float* P, const uint32_t* Order, const float* N
 }
 
 TightScratch::~TightScratch() {
-  if (boxes != nullptr && cudaFreeAsync(boxes, stream) != cudaSuccess) cudaGetLastError();
+  if (boxes == nullptr) return;
+  const OtherCaptures undisturbed;
+  if (cudaFreeAsync(boxes, stream) != cudaSuccess) cudaGetLastError();
 }
 
 }  // namespace arbor
