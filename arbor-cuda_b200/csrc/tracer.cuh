@@ -133,6 +133,8 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
   // distances as one multiply-add each.
   const f3 far = max3(mk(fabsf(lo.x - lro.x), fabsf(lo.y - lro.y), fabsf(lo.z - lro.z)), mk(fabsf(hi.x - lro.x), fabsf(hi.y - lro.y), fabsf(hi.z - lro.z)));
   const float d = length3(far);
+  // (a surface beyond kFar would be a hit after all)
+  if (r.lfound == kMissCounts && !(d < 0.99f * kFar)) r.lfound = kInOrder;
   float m = c.tight.rel * d + c.tight.abs;
   float slack = 0.0f;
   r.boxes = 0;

@@ -315,3 +315,16 @@ def test_ground_beyond_the_farthest_distance(emu, distance):
         got, want, _ = s.both(rays, wind=wind)
         assert (want[:, 0] > FAR).sum() >= 20 and ((want[:, 0] == FAR) & (want[:, 1] >= 0)).sum() >= 5
         same(got, want)
+
+
+@pytest.mark.parametrize("distance", [9.0e4, 1.2e5, 3.0e5])
+def test_surfaces_beyond_the_farthest_distance(emu, distance):
+    """A scene 4 km across, farther away than t = 100000, before a ground that
+    is farther still: its hits lie beyond the tests' "no hit" value."""
+    s = Scene(emu, [stone(0.0, 500.0, 0.0, 2000.0), stone(1500.0, 900.0, 0.0, 900.0)])
+    rays = rays_at((0.0, 500.0, 0.0), 2500.0, distance, 128, 7)
+    rays[:, 6] = np.where(np.arange(128) % 2, FAR, distance + 1.0e5)
+    for refine in (True, False):
+        got, want, _ = s.both(rays, refine=refine, against="emu_in_order")
+        assert (want[:, 1] >= 0).sum() >= 10
+        same(got, want)
