@@ -61,6 +61,7 @@ constexpr size_t kTightBytes = sizeof(uint32_t) * kTightWords;
 static_assert(kTightWords % 4 == 0, "16-byte aligned groups in every scene");
 constexpr float kTightRel = 1.3e-3f;
 constexpr float kTightMost = 0.10f;  // the widest margin at which the tight boxes are the smaller ones
+constexpr float kTightTaper = 0.25f;  // steepest taper the margin covers (wood the library grows: 0.143, its petioles: 0.02)
 constexpr float kSwing = 0.156f;  // wind's largest turn per unit (0.11 + 0.045 radians, rounded up)
 
 struct TightPart {
@@ -101,14 +102,19 @@ __device__ __forceinline__ void add_axis(float c, float a, float b, float& lo, f
 // blade and petiole in still air, and returns the leaf's reach (0: not a leaf).
 // -1: the surface is not known to lie inside the box - a leaf wider than it is
 // long or curled up beyond its cube, a frame that is not orthonormal, a size
-// that is negative or not finite, an unknown type.  A ray can then pass the box
+// that is negative or not finite, an unknown type, a taper so steep that the
+// cone's test goes wrong by more than the margin (its radius and the root's
+// terms grow with the taper times the distance).  A ray can then pass the box
 // in one place and meet the surface in another, and which hit counts depends on
 // the order: the scene is traversed in the fixed one.
 __device__ __forceinline__ float tighten_record(const float* P, int id, float4& lo, float4& hi) {
   const float4 r0 = ldg4(P, id * 6), r1 = ldg4(P, id * 6 + 1), r2 = ldg4(P, id * 6 + 2), r3 = ldg4(P, id * 6 + 3), r4 = ldg4(P, id * 6 + 4);
   const int type = (int)r0.w;
   if (!(lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z)) return -1.0f;
-  if (type == 0) return r1.w >= 0.0f && r2.w >= 0.0f ? 0.0f : -1.0f;
+  if (type == 0) {
+    const f3 ab = xyz(r1) - xyz(r0);
+    return r1.w >= 0.0f && r2.w >= 0.0f && fabsf(r2.w - r1.w) <= kTightTaper * length3(ab) ? 0.0f : -1.0f;
+  }
   if (type != 1) return type == 2 ? 0.0f : -1.0f;
   const f3 o = xyz(r0), u = xyz(r1), v = xyz(r2), n = xyz(r3);
   const float len = r1.w, width = r2.w, stem = r4.x;
@@ -117,6 +123,7 @@ __device__ __forceinline__ float tighten_record(const float* P, int id, float4& 
   const float x1 = stem + len + 0.002f, w = fmaxf(width, 0.002f) + 0.0005f;
   const float reach = sqrtf(x1 * x1 + w * w + 0.0045f);  // 0.067^2 across
   if (!(g < 1.0e-4f) || !(len >= 0.0f) || !(stem >= 0.0f) || !(width >= 0.0f) || !(reach < 1.0e3f)) return -1.0f;
+  if (stem > 0.0f && 0.00045f > kTightTaper * stem) return -1.0f;  // (without a stem the petiole is two balls)
   // Across the blade its height (leaf_height for 0 <= q <= 1, |v| <= width: curl,
   // twist, 9 mm of cupping, the 1.2 mm rib, the solve's tolerance) within the
   // clip box's -0.035 .. 0.065, and the petiole's radius.

@@ -328,3 +328,24 @@ def test_surfaces_beyond_the_farthest_distance(emu, distance):
         got, want, _ = s.both(rays, refine=refine, against="emu_in_order")
         assert (want[:, 1] >= 0).sum() >= 10
         same(got, want)
+
+
+@pytest.mark.parametrize("kind", ["petioles", "wood"])
+@pytest.mark.parametrize("refine", [True, False])
+def test_steep_tapers(emu, kind, refine):
+    """Petioles a hundredth as long as they are thick, wood whose radius falls
+    faster than it is long: the cone's test reports hits far off the surface,
+    and they count as they do in the fixed order."""
+    r = np.random.RandomState(11)
+    recs = []
+    for _ in range(120):
+        p = 0.06 * (r.random(3) - 0.5) + (0.0, 0.06, 0.0)
+        if kind == "petioles":
+            u, v, w = (x / np.linalg.norm(x) for x in np.linalg.qr(r.standard_normal((3, 3)))[0].T)
+            recs.append(leaf(*p, 1.0e-3, 4.0e-4, stem=10.0 ** r.uniform(-5.5, -4.0), curl=1.0e-4, twist=0.1, frame=(u, v, w)))
+        else:
+            recs.append(wood(p, p + 1.0e-4 * r.standard_normal(3), 3.0e-3, 1.0e-3))
+    s = Scene(emu, recs)
+    got, want, _ = s.both(rays_at((0.0, 0.06, 0.0), 0.03, 6.0, 800, 12, best=FAR if refine else 36.0), refine=refine, against="emu_in_order")
+    assert (want[:, 1] >= 0).sum() >= 50
+    same(got, want)
