@@ -373,8 +373,9 @@ __device__ __forceinline__ void conv_stage_weights(const ConvArgs& a, int c0, ui
 // The MMAs of one 16-channel step (A descriptor da) of one tap column on the
 // accumulators of COUNT successive output rows at tmem columns acc: weights
 // db of the first row's dy, the other rows' behind them.  At most 256 columns
-// at a time.  (One thread issues them all: counts are compile-time constants,
-// a loop over them took as long as the MMAs.)
+// at a time.  (One thread issues them all, and counts are compile-time
+// constants: with descriptors computed in the loop an MMA took 179 cycles at any
+// N.)
 template <int N, int COUNT>
 __device__ __forceinline__ void umma_rows(uint32_t acc, uint64_t da, uint64_t db, bool accumulate) {
   constexpr int MAX = 256 / N;
@@ -439,9 +440,9 @@ __device__ __forceinline__ void conv_ctl_end(ConvCtl<S, B>& c, int cols, bool ok
 // An input row feeds three output rows, one per dy.  Their accumulators are
 // neighbours in TMEM (a ring of B blocks of N columns) and the three dy's
 // weights neighbours in shared memory, so one MMA of 3 N columns does all
-// three: what an MMA costs here is reading its A operand (128 pixels x 16
-// channels: measured 150-200 cycles for N = 32 .. 96), and a row's A is read 3
-// times, once per dx, instead of 9.  The products of an output still come in
+// three: an MMA of 128 pixels x 16 channels takes a flat 52 cycles up to N = 64,
+// 57 for 96 and N / 2 beyond, so three rows of N = 32 cost as much as one.  The
+// products of an output still come in
 // the order dy, dx, channel step.
 template <int N, int CIN, int S, int B>
 constexpr int conv_row_smem_bytes() {

@@ -9,6 +9,10 @@ source performs for it (Arbor.cu line cited per weight), counting every
 add, subtract, multiply, divide, square root, min, max, abs, floor and each
 call of a transcendental function (sin, cos, exp, pow, atan2) as one
 operation.  Integer hashing, conversions and comparisons are not counted.
+The counts are those of the reference's order of visits and tests: the passes
+reach the same result over tighter boxes with far fewer (`work` in the bench
+line says so), so `achieved` is the reference algorithm's work over our time and
+not the rate at which the kernels issue.
 
 Peak: the arithmetic is compiled without FMA contraction (the reference's
 rounding), so the usable FP32 rate is one operation per lane per cycle:
@@ -73,16 +77,17 @@ def flops(counts: dict) -> int:
     return int(sum(WEIGHTS[k] * counts[k] for k in EVENTS))
 
 
-# DRAM traffic per unit, measured with ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum) on one 960x544 launch of the forest walk's first
-# frame (seed 7, cold caches): the trace kernel moved 5.33 MB for 522,240
-# primary rays, the shadow pass of shadePixels 20.31 MB for 522,240 pixels
-# (before the tight boxes; those add 0.8 MB per launch).
-# The 5.7 MB scene stays in L2, so the traffic grows with the pixel count;
-# bench lines scale these to their launch.
-TRACE_DRAM_BYTES_PER_RAY = 10.2
-SHADOW_DRAM_BYTES_PER_PIXEL = 38.9
-TRAFFIC_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 960x544 forest launch, scaled by units to this launch"
+# DRAM traffic of a launch, measured with ncu (dram__bytes_read.sum +
+# dram__bytes_write.sum, cold caches) on forest frames with sun shadows at
+# 960x540 and 1920x1080.  The trace moved 9.14 and 10.93 MB: the 5.7 MB scene and
+# its tight boxes once, and little of the Hit image, which stays in L2.  The
+# shadow pass moved 16.6 and 71.8 MB: Hit, Linear and Guide as they leave L2.
+# Both grow linearly between the two sizes; the bench lines take them so.
+TRACE_DRAM_BYTES, TRACE_DRAM_BYTES_PER_RAY = 8.55e6, 1.15
+SHADOW_DRAM_BYTES, SHADOW_DRAM_BYTES_PER_PIXEL = -1.75e6, 35.4
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of forest launches at 960x540 and 1920x1080, linear in the pixels between "
+                  "them")
+WORK_SOURCE = "tests of the reference's traversal order (count.cu); this pass makes fewer"
 
 
 def roofline_entry(kernel: str, counts: dict, pixels: int, ms: float, fp32_peak_tops: float, sm_clock_mhz: float,
@@ -97,7 +102,7 @@ def roofline_entry(kernel: str, counts: dict, pixels: int, ms: float, fp32_peak_
         "kernel": kernel, "bound": "fp32", "achieved": round(achieved, 3), "peak": round(fp32_peak_tops, 2),
         "unit": "TFLOP/s", "frac": round(achieved / fp32_peak_tops, 4), "traffic": traffic,
         **({"traffic_source": traffic_source} if traffic is not None else {}),
-        "algorithmic_flops": ops, "flops_per_pixel": round(ops / pixels, 1),
+        "work": WORK_SOURCE, "algorithmic_flops": ops, "flops_per_pixel": round(ops / pixels, 1),
         "events_per_pixel": {k: round(v / pixels, 3) for k, v in counts.items() if v},
         "peak_source": f"derived: 148 SM x 128 FP32 lanes x {sm_clock_mhz:.0f} MHz measured SM clock, one non-fused op per lane per "
                        "cycle (no FP32 peak in MEASURED_PEAKS.json)",
@@ -107,7 +112,7 @@ def roofline_entry(kernel: str, counts: dict, pixels: int, ms: float, fp32_peak_
 
 def trace_roofline(ab, fr, torch, ms_trace: float, fp32_peak_tops: float, sm_clock_mhz: float) -> dict:
     counts = count_events(ab, fr.P, fr.Nodes, fr.Order, fr.C, fr.w, fr.h, fr.spec["single_tree"], torch)
-    traffic = None if fr.spec["single_tree"] else int(TRACE_DRAM_BYTES_PER_RAY * fr.w * fr.h)
+    traffic = None if fr.spec["single_tree"] else int(TRACE_DRAM_BYTES + TRACE_DRAM_BYTES_PER_RAY * fr.w * fr.h)
     return roofline_entry("tracePixels", counts, fr.w * fr.h, ms_trace, fp32_peak_tops, sm_clock_mhz, traffic,
                           TRAFFIC_SOURCE + " (trace_pool_kernel)")
 
@@ -115,6 +120,6 @@ def trace_roofline(ab, fr, torch, ms_trace: float, fp32_peak_tops: float, sm_clo
 def shade_roofline(ab, fr, torch, ms_shade: float, fp32_peak_tops: float, sm_clock_mhz: float) -> dict:
     counts = count_events(ab, fr.P, fr.Nodes, fr.Order, fr.C, fr.w, fr.h, fr.spec["single_tree"], torch, Hit=fr.Hit)
     shadows = bool(fr.spec.get("shadows")) and not fr.spec["single_tree"]
-    traffic = int(SHADOW_DRAM_BYTES_PER_PIXEL * fr.w * fr.h) if shadows else None
+    traffic = max(0, int(SHADOW_DRAM_BYTES + SHADOW_DRAM_BYTES_PER_PIXEL * fr.w * fr.h)) if shadows else None
     return roofline_entry("shadePixels", counts, fr.w * fr.h, ms_shade, fp32_peak_tops, sm_clock_mhz, traffic,
                           TRAFFIC_SOURCE + " (shadow_pool_kernel; the compose pass, 64 B/px, is not included)")

@@ -745,7 +745,7 @@ def run_batch(args, rank: int, world: int, local_rank: int) -> None:
             "autotune": {"chosen": best, "sample_views": args.tune_views, "seconds": round(tune_s, 2),
                          "ms_per_config": {f"tw{tw}_ctas{c}_order{o}_q{q}": round(table[i], 3)
                                            for i, (tw, c, o, q) in enumerate((tw, c, o, q) for tw in (16, 32) for c in (1, 2)
-                                                                             for o in (0, 1) for q in (4, 8))}},
+                                                                             for o in (0, 1) for q in (12, 16))}},
             "phases_ms": {"setup": round(ms_setup, 4), "trace": round(ms_trace, 4), "shade": round(ms_shade, 4),
                           "filter_resolve": round(ms_filter, 4)},
             "roofline": r_trace if ms_trace >= ms_shade else r_shade, "roofline_trace": r_trace, "roofline_shade": r_shade,
