@@ -1,6 +1,6 @@
 """What the library remembers of a device (shared-memory opt-ins, the number of
-multiprocessors) is kept per device and is safe between threads.  (Not tested on
-a second GPU: every run here has one.)"""
+multiprocessors) is kept per device and is safe between threads.  (The library
+itself has not run on a second GPU.)"""
 import ctypes
 import glob
 import os
