@@ -121,7 +121,7 @@ __device__ __forceinline__ void batch_view(const BatchView* __restrict__ views, 
 template <bool kShadow, int Q>
 __device__ __noinline__ void batch_view_in_order(const BatchView* __restrict__ views, const Camera* __restrict__ cams,
                                                  const Instance* __restrict__ insts, int v, int* __restrict__ queues, OrderBatchOf<Q>* b) {
-  batch_view<kShadow>(views, cams, insts, v, queues, TightView{nullptr, 0.0f, 0.0f}, *b);
+  batch_view<kShadow>(views, cams, insts, v, queues, TightView{nullptr, 0.0f, 0.0f, 0.0f}, *b);
 }
 
 // The pass over every listed view.  Each CTA walks the views in

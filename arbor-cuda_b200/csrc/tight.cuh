@@ -27,12 +27,14 @@
 // Pruning is by the widened box's entry, which no reported t can precede.
 //
 // The margin grows with the distance and the boxes' own size does not: from
-// about 80 m on a widened tight box is larger than the box in Nodes, whose test
-// needs no margin.  So the boxes of Nodes are stored too, the same way, and a
-// primary ray takes, tree by tree, the tight ones up to a margin of kTightMost
+// about 80 m on a widened tight box of a grown tree is larger than the box in
+// Nodes, whose test needs no margin.  So the boxes of Nodes are stored too, the
+// same way, and a primary ray takes, tree by tree, the tight ones up to a margin
+// of kTightMost times the largest leaf's reach (0.29 m in a grown scene: 0.10 m)
 // and those of Nodes beyond (1080p trace 6.4 -> 5.4 ms, 5.7 with the line at
 // 0.05 m and 5.6 at 0.20; small frames that look along the canopy were up to 1.7
-// times slower with tight boxes at every distance).
+// times slower with tight boxes at every distance; a forest of trees a tenth as
+// large 2.6 times slower with the line at 0.10 m whatever the leaves).
 //
 // The boxes are stored 16 bits a coordinate, on a grid over the root's box and
 // rounded outward: the four nodes 4g .. 4g + 3 that a traversal step tests
@@ -60,7 +62,7 @@ constexpr int kTightWords = kTightGrid + 8;              // words per scene
 constexpr size_t kTightBytes = sizeof(uint32_t) * kTightWords;
 static_assert(kTightWords % 4 == 0, "16-byte aligned groups in every scene");
 constexpr float kTightRel = 1.3e-3f;
-constexpr float kTightMost = 0.10f;  // the widest margin at which the tight boxes are the smaller ones
+constexpr float kTightMost = 0.345f;  // the widest margin at which the tight boxes are the smaller ones, in reaches
 constexpr float kTightTaper = 0.25f;  // steepest taper the margin covers (wood the library grows: 0.143, its petioles: 0.02)
 constexpr float kSwing = 0.156f;  // wind's largest turn per unit (0.11 + 0.045 radians, rounded up)
 
@@ -250,6 +252,7 @@ static_assert(kTightLeaves / 2 == 256, "one thread per node of the widest inner 
 struct TightView {
   const uint32_t* T;  // the boxes of its scene(s), kTightWords each; null: Nodes, in a fixed order (orderbatch.cuh)
   float rel, abs;     // the boxes' margin: rel x D + abs
+  float most;         // the widest margin at which primary rays take them
 };
 // Largest swing of a leaf under `wind` whose reach is `reach`.
 __device__ __forceinline__ float swing_margin(float wind, float reach) { return fminf(fabsf(wind) * kSwing, 2.0f) * reach; }
@@ -258,15 +261,15 @@ __device__ __forceinline__ float swing_margin(float wind, float reach) { return 
 __device__ __forceinline__ TightView tight_view_warp(const uint32_t* T, float wind) {
   const int lane = threadIdx.x & 31;
   const float a = __uint_as_float(__ldg(T + kTightReach + lane)), b = __uint_as_float(__ldg(T + kTightReach + 32 + lane));
-  if (__any_sync(0xffffffffu, !(a >= 0.0f) || !(b >= 0.0f))) return {nullptr, 0.0f, 0.0f};
+  if (__any_sync(0xffffffffu, !(a >= 0.0f) || !(b >= 0.0f))) return {nullptr, 0.0f, 0.0f, 0.0f};
   const int reach = __reduce_max_sync(0xffffffffu, __float_as_int(fmaxf(a, b)));
-  return {T, kTightRel, swing_margin(wind, __int_as_float(reach))};
+  return {T, kTightRel, swing_margin(wind, __int_as_float(reach)), kTightMost * __int_as_float(reach)};
 }
 // A block: the view of n scenes' boxes T (null: none were made).  Every thread
 // calls it.
 __device__ __forceinline__ TightView tight_view_block(const uint32_t* T, int n, float wind) {
   __shared__ int reach;
-  if (T == nullptr) return {nullptr, 0.0f, 0.0f};
+  if (T == nullptr) return {nullptr, 0.0f, 0.0f, 0.0f};
   if (threadIdx.x == 0) reach = 0;
   __syncthreads();
   bool bad = false;
@@ -275,8 +278,8 @@ __device__ __forceinline__ TightView tight_view_block(const uint32_t* T, int n, 
     bad |= !(r >= 0.0f);
     atomicMax(&reach, __float_as_int(r));
   }
-  if (__syncthreads_or(bad)) return {nullptr, 0.0f, 0.0f};
-  return {T, kTightRel, swing_margin(wind, __int_as_float(reach))};
+  if (__syncthreads_or(bad)) return {nullptr, 0.0f, 0.0f, 0.0f};
+  return {T, kTightRel, swing_margin(wind, __int_as_float(reach)), kTightMost * __int_as_float(reach)};
 }
 
 }  // namespace arbor

@@ -138,7 +138,7 @@ __device__ __forceinline__ bool enter_tree(const TraceCtx& c, Ray& r, WB& b, int
   float m = c.tight.rel * d + c.tight.abs;
   float slack = 0.0f;
   r.boxes = 0;
-  if (c.refine && m > kTightMost) {  // (a shadow segment is 36 m at most; its pruning has no slack)
+  if (c.refine && m > c.tight.most) {  // (a shadow segment is 36 m at most; its pruning has no slack)
     // The boxes are not widened, but a hit may still come before its box by
     // the margin: pruning allows for it.
     slack = m;

@@ -349,3 +349,30 @@ def test_steep_tapers(emu, kind, refine):
     got, want, _ = s.both(rays_at((0.0, 0.06, 0.0), 0.03, 6.0, 800, 12, best=FAR if refine else 36.0), refine=refine, against="emu_in_order")
     assert (want[:, 1] >= 0).sum() >= 50
     same(got, want)
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.1])
+def test_small_trees_far_away_are_not_searched_whole(emu, scenes, scale):
+    """A grown tree, and one a tenth as large, from as far as the margin is wide
+    beside a leaf: the loads stay below twice the fixed order's, which tests the
+    boxes of Nodes (a tenth as large, tight boxes widened by three leaves: 3
+    times)."""
+    src = scenes(7)
+    s = Grown(emu, src, lambda N: None)
+    P = s.P.reshape(CAPACITY, 24)
+    kind = P[:, 3].copy()
+    P[:, [0, 1, 2, 7, 11]] *= np.float32(scale)
+    P[kind != 1, 4:7] *= np.float32(scale)
+    P[kind == 1, 16:18] *= np.float32(scale)
+    P[kind == 0, 16] *= np.float32(scale)
+    P[kind == 0, 18] *= np.float32(scale)
+    emu.emu_leaf_nodes(_p(s.P), _p(s.Order), _p(s.Nodes))
+    assert emu.emu_boxes(_p(s.P), _p(s.Order), _p(s.Nodes), _p(s.T)) == 0
+    rays = rays_at((0.0, 5.5 * scale, 0.0), 3.0 * scale, 70.0, 200, 1)
+    got, want, regular = s.both(rays, against="emu_in_order")
+    batch = emu.emu_loads()
+    same(got, want)
+    s.T = None
+    s.both(rays, against="emu_in_order")
+    print(f"[scale {scale}] {batch} loads, in order {emu.emu_loads()}")
+    assert regular == 1 and batch < 2 * emu.emu_loads()
