@@ -116,8 +116,14 @@ __device__ __forceinline__ void batch_view(const BatchView* __restrict__ views, 
     block_drive(c, r, b, policy, pool);
   }
 }
+// What a view's pass traverses.
+template <bool kShadow>
+__device__ __forceinline__ TightView batch_tight(const BatchView* __restrict__ views, int v, float wind) {
+  const TightView tight = tight_view_warp(views[v].T, wind);
+  return kShadow ? tight : primary_view(tight, 1, kForestFar);
+}
 // The same in a fixed order, for a scene whose Nodes the caller has changed
-// (arbor_batch_view_buffers).
+// (arbor_batch_view_buffers) and primary rays in a storm (primary_view).
 template <bool kShadow, int Q>
 __device__ __noinline__ void batch_view_in_order(const BatchView* __restrict__ views, const Camera* __restrict__ cams,
                                                  const Instance* __restrict__ insts, int v, int* __restrict__ queues, OrderBatchOf<Q>* b) {
@@ -135,12 +141,12 @@ __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* 
   using BB = BlockBatchOf<Q>;
   static_assert(sizeof(OrderBatchOf<Q>) <= sizeof(BB), "in the other batch's memory");
   extern __shared__ float4 batch_smem[];
-  bool rest = false;  // (the changed scenes' views in a loop of their own: with the call in this one it ran 5 % slower)
+  bool rest = false;  // (the views in a fixed order in a loop of their own: with the call in this one it ran 5 % slower)
   for (int i = 0; i < n_list; i++) {
     const int v = __ldg(list + i);
     const Camera& cam = cams[v];
     if (kShadow && !(cam.shadows > 0.5f)) continue;
-    const TightView tight = tight_view_warp(views[v].T, cam.wind);  // uniform
+    const TightView tight = batch_tight<kShadow>(views, v, cam.wind);  // uniform
     if (tight.T != nullptr)
       batch_view<kShadow>(views, cams, insts, v, queues, tight, *reinterpret_cast<BB*>(batch_smem));
     else
@@ -148,7 +154,7 @@ __global__ void __launch_bounds__(kBlock, 2) batch_pool_kernel(const BatchView* 
   }
   for (int i = 0; rest && i < n_list; i++) {
     const int v = __ldg(list + i);
-    if ((!kShadow || cams[v].shadows > 0.5f) && tight_view_warp(views[v].T, 0.0f).T == nullptr)
+    if ((!kShadow || cams[v].shadows > 0.5f) && batch_tight<kShadow>(views, v, cams[v].wind).T == nullptr)
       batch_view_in_order<kShadow>(views, cams, insts, v, queues, reinterpret_cast<OrderBatchOf<Q>*>(batch_smem));
   }
 }

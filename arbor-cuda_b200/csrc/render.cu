@@ -57,7 +57,8 @@ __global__ void __launch_bounds__(kBlock, 2) trace_pool_kernel(const float* __re
   if (threadIdx.x == 0) next = 0;
   block_setup(C, cam, nullptr, false, nullptr);
   const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, T, 1, smem) : nullptr;
-  const TightView tight = tight_view_block(T, 1, cam.wind);
+  const TightView boxes = tight_view_block(T, 1, cam.wind);
+  const TightView tight = primary_view(boxes, 1, kForestScene ? kForestFar : tree_far(boxes, cam.ro));
   const TraceCtx c{P, Nodes, Order, inst, tight, cam.c14 / (float)height, cam.time, cam.wind, true, kForestScene};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(kBlock, 2) trace_species_kernel(const float* _
   for (int t = threadIdx.x; t < kForest; t += blockDim.x) of[t] = map.of[t];
   block_setup(C, cam, nullptr, false, nullptr);
   const Instance* inst = pass_instances(trig, cam.ws, T, n_scenes, smem);
-  const TightView tight = tight_view_block(T, n_scenes, cam.wind);
+  const TightView tight = primary_view(tight_view_block(T, n_scenes, cam.wind), n_scenes, kForestFar);
   const TraceCtx c{P, Nodes, Order, inst, tight, cam.c14 / (float)height, cam.time, cam.wind, true, true, true, of};
   const int bx = (width + 7) / 8;
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};

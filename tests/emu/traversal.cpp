@@ -85,6 +85,19 @@ long emu_trace(const float* P, const uint32_t* Order, const float* Nodes, const 
   return emu::bad_loads;
 }
 
+// Whether primary rays of a scene take its boxes (1) or the fixed order (0):
+// from `eye` for the single tree, anywhere in a forest without.
+int emu_primary_takes_boxes(const uint32_t* T, float wind, const float* eye) {
+  emu::buffers = {{(const char*)T, (const char*)(T + kTightWords)}};
+  int takes = -1;
+  emu::run(kThreads, 0, 1, [&] {
+    const TightView boxes = tight_view_block(T, 1, wind);
+    const TightView v = primary_view(boxes, 1, eye ? tree_far(boxes, mk(eye[0], eye[1], eye[2])) : kForestFar);
+    if (threadIdx.x == 0) takes = v.T != nullptr;
+  });
+  return takes;
+}
+
 // The same rays one by one, each tree by tree_in_order.
 void emu_in_order(const float* P, const uint32_t* Order, const float* Nodes, const Instance* inst, const float* rays, int n, float cone,
                   float time, float wind, int refine, float* out) {

@@ -351,14 +351,9 @@ def test_steep_tapers(emu, kind, refine):
     same(got, want)
 
 
-@pytest.mark.parametrize("scale", [1.0, 0.1])
-def test_small_trees_far_away_are_not_searched_whole(emu, scenes, scale):
-    """A grown tree, and one a tenth as large, from as far as the margin is wide
-    beside a leaf: the loads stay below twice the fixed order's, which tests the
-    boxes of Nodes (a tenth as large, tight boxes widened by three leaves: 3
-    times)."""
-    src = scenes(7)
-    s = Grown(emu, src, lambda N: None)
+def scaled(emu, scene, scale):
+    """A grown scene with every length times `scale`."""
+    s = Grown(emu, scene, lambda N: None)
     P = s.P.reshape(CAPACITY, 24)
     kind = P[:, 3].copy()
     P[:, [0, 1, 2, 7, 11]] *= np.float32(scale)
@@ -368,6 +363,16 @@ def test_small_trees_far_away_are_not_searched_whole(emu, scenes, scale):
     P[kind == 0, 18] *= np.float32(scale)
     emu.emu_leaf_nodes(_p(s.P), _p(s.Order), _p(s.Nodes))
     assert emu.emu_boxes(_p(s.P), _p(s.Order), _p(s.Nodes), _p(s.T)) == 0
+    return s
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.1])
+def test_small_trees_far_away_are_not_searched_whole(emu, scenes, scale):
+    """A grown tree, and one a tenth as large, from as far as the margin is wide
+    beside a leaf: the loads stay below twice the fixed order's, which tests the
+    boxes of Nodes (a tenth as large, tight boxes widened by three leaves: 3
+    times)."""
+    s = scaled(emu, scenes(7), scale)
     rays = rays_at((0.0, 5.5 * scale, 0.0), 3.0 * scale, 70.0, 200, 1)
     got, want, regular = s.both(rays, against="emu_in_order")
     batch = emu.emu_loads()
@@ -376,3 +381,15 @@ def test_small_trees_far_away_are_not_searched_whole(emu, scenes, scale):
     s.both(rays, against="emu_in_order")
     print(f"[scale {scale}] {batch} loads, in order {emu.emu_loads()}")
     assert regular == 1 and batch < 2 * emu.emu_loads()
+
+
+@pytest.mark.parametrize("scale,wind,distance,boxes", [
+    (1.0, 0.0, None, 1), (1.0, 0.6, None, 1), (1.0, 3.0, None, 1), (1.0, 8.0, None, 0), (0.5, 0.0, None, 1), (0.2, 0.0, None, 0),
+    (1.0, 0.0, 3.0, 1), (1.0, 0.0, 300.0, 1), (1.0, 8.0, 3.0, 1), (1.0, 8.0, 300.0, 0), (1.0, 0.0, 600.0, 0),
+    (0.2, 0.0, 3.0, 1), (0.2, 3.0, 10.0, 1), (0.2, 0.0, 300.0, 0), (0.1, 0.0, 30.0, 1), (0.1, 0.0, 100.0, 0)])
+def test_what_primary_rays_traverse(emu, scenes, scale, wind, distance, boxes):
+    """The faster of tight boxes and fixed order, as measured (tight.cuh), for a
+    forest (distance None) and the single tree."""
+    s = scaled(emu, scenes(7), scale)
+    eye = None if distance is None else np.array([0.0, 5.0 * scale, distance], np.float32)
+    assert emu.emu_primary_takes_boxes(_p(s.T), ctypes.c_float(wind), _p(eye)) == boxes
