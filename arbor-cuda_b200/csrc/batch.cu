@@ -120,10 +120,10 @@ __device__ __forceinline__ void batch_view(const BatchView* __restrict__ views, 
 template <bool kShadow>
 __device__ __forceinline__ TightView batch_tight(const BatchView* __restrict__ views, int v, float wind) {
   const TightView tight = tight_view_warp(views[v].T, wind);
-  return kShadow ? tight : primary_view(tight, 1, kForestFar);
+  return kShadow ? shadow_view(tight, wind) : primary_view(tight, 1, kForestFar);
 }
 // The same in a fixed order, for a scene whose Nodes the caller has changed
-// (arbor_batch_view_buffers) and primary rays in a storm (primary_view).
+// (arbor_batch_view_buffers) and views in a storm (primary_view, shadow_view).
 template <bool kShadow, int Q>
 __device__ __noinline__ void batch_view_in_order(const BatchView* __restrict__ views, const Camera* __restrict__ cams,
                                                  const Instance* __restrict__ insts, int v, int* __restrict__ queues, OrderBatchOf<Q>* b) {

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kBlock, 2) shadow_pool_kernel(const float* __r
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
   stage_shadows(cam, Hit, Linear, Guide, pool);
   const Instance* inst = kForestScene ? pass_instances(trig, cam.ws, T, 1, smem) : nullptr;
-  const TightView tight = tight_view_block(T, 1, cam.wind);
+  const TightView tight = shadow_view(tight_view_block(T, 1, cam.wind), cam.wind);
   const TraceCtx c{P, Nodes, Order, inst, tight, 0.0001f, cam.time, cam.wind, false, kForestScene};
   staged_shadow_pool(c, smem.batch, Guide, Linear, pool);
 }
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kBlock, 2) shadow_species_kernel(const float* 
   const PixelPool pool{&next, width, height, bx, bx * ((height + 3) / 4)};
   stage_shadows(cam, Hit, Linear, Guide, pool);
   const Instance* inst = pass_instances(trig, cam.ws, T, n_scenes, smem);
-  const TightView tight = tight_view_block(T, n_scenes, cam.wind);
+  const TightView tight = shadow_view(tight_view_block(T, n_scenes, cam.wind), cam.wind);
   const TraceCtx c{P, Nodes, Order, inst, tight, 0.0001f, cam.time, cam.wind, false, true, true, of};
   staged_shadow_pool(c, smem.batch, Guide, Linear, pool);
 }

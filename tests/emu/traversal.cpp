@@ -98,6 +98,17 @@ int emu_primary_takes_boxes(const uint32_t* T, float wind, const float* eye) {
   return takes;
 }
 
+// Whether its shadow segments do.
+int emu_shadow_takes_boxes(const uint32_t* T, float wind) {
+  emu::buffers = {{(const char*)T, (const char*)(T + kTightWords)}};
+  int takes = -1;
+  emu::run(kThreads, 0, 1, [&] {
+    const TightView v = shadow_view(tight_view_block(T, 1, wind), wind);
+    if (threadIdx.x == 0) takes = v.T != nullptr;
+  });
+  return takes;
+}
+
 // The same rays one by one, each tree by tree_in_order.
 void emu_in_order(const float* P, const uint32_t* Order, const float* Nodes, const Instance* inst, const float* rays, int n, float cone,
                   float time, float wind, int refine, float* out) {

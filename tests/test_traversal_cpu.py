@@ -393,3 +393,12 @@ def test_what_primary_rays_traverse(emu, scenes, scale, wind, distance, boxes):
     s = scaled(emu, scenes(7), scale)
     eye = None if distance is None else np.array([0.0, 5.0 * scale, distance], np.float32)
     assert emu.emu_primary_takes_boxes(_p(s.T), ctypes.c_float(wind), _p(eye)) == boxes
+
+
+@pytest.mark.parametrize("leaves,wind,boxes", [(1, 0.0, 1), (1, 0.6, 1), (1, -2.0, 1), (1, 3.0, 0), (1, -8.0, 0), (1, float("inf"), 0),
+                                               (1, float("nan"), 0), (0, 8.0, 1)])
+def test_what_shadow_segments_traverse(emu, leaves, wind, boxes):
+    """The faster of tight boxes and fixed order, as measured (tight.cuh): the
+    boxes in a breeze, or where nothing swings."""
+    s = Scene(emu, [stone(0.0, 1.0, 0.0, 0.3), leaf(0.0, 1.0, 0.0, 0.15, 0.07) if leaves else stone(0.2, 1.0, 0.0, 0.1)])
+    assert emu.emu_shadow_takes_boxes(_p(s.T), ctypes.c_float(wind)) == boxes
