@@ -69,3 +69,25 @@ def test_batch_scene_changed_through_its_buffers(cuda, queue):
                 assert np.array_equal(np.ascontiguousarray(got[k]).view(np.uint32), np.ascontiguousarray(want[k]).view(np.uint32)), f"view {v} {k}"
     finally:
         batch.close()
+
+
+@pytest.mark.parametrize("wind", [3.0, 8.0, 30.0])
+def test_batch_in_a_storm(cuda, wind):
+    """Views whose wind sends the shadow pass, or both passes, to the fixed
+    order, beside one in still air."""
+    import gpu_util
+
+    views = []
+    for v, (w, h) in enumerate(((320, 180), (97, 61), (160, 90))):
+        C = workloads.view_pose_state((7, 1788)[v % 2], w, h, 11.0, -23.0, 0.7, 0.12)
+        C[8], C[11] = 3.25, 0.0 if v == 1 else wind
+        views.append((v % 2, w, h, C))
+    batch = Batch(views)
+    try:
+        batch.call("arbor_batch_render")
+        for v in range(len(views)):
+            got, want = batch.images(v), single_image(cuda, gpu_util, batch, v)
+            for k in ("Hit", "Linear", "Guide", "Filtered", "Pixels"):
+                assert np.array_equal(np.ascontiguousarray(got[k]).view(np.uint32), np.ascontiguousarray(want[k]).view(np.uint32)), f"view {v} {k}"
+    finally:
+        batch.close()
